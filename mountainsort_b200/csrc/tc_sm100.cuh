@@ -179,6 +179,16 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
     }
 }
 
+// The same for waits that are usually well under a microsecond: probes without
+// suspending first (a suspended thread takes longer to wake than such a wait
+// lasts), then the bounded wait.
+__device__ __forceinline__ bool mbar_wait_cluster_spin(uint64_t* bar, uint32_t parity, int* err) {
+#pragma unroll 1
+    for (int k = 0; k < 256; k++)
+        if (mbar_try_wait_cluster(bar, parity)) return true;
+    return mbar_wait_cluster(bar, parity, err);
+}
+
 __device__ __forceinline__ void bulk_commit_group() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 
 // Waits until at most N bulk groups of this thread are still reading shared memory.

@@ -13,7 +13,9 @@
 //       so the result agrees with the reference's double sum of float
 //       products to ~1e-10 relative.  Partial tiles are reduced in a fixed
 //       order: repeat runs are bit-identical.
-//   pca_cluster   the reference's power iteration, FP64, one thread-block
+//   pca_reg       the reference's power iteration, FP64, the working matrix in
+//       the registers of one CTA or one cluster of 16 (up to 512 channels)
+//   pca_cluster   the same for more channels, one thread-block
 //       cluster: the working matrix XXtw is split by rows across the CTAs'
 //       shared memory (global memory beyond what fits); each matvec result
 //       is broadcast to every CTA through distributed shared memory, one
@@ -32,6 +34,7 @@
 #include <string>
 
 #include "common.cuh"
+#include "div_by.cuh"
 #include "ms3gpu.h"
 #include "tc_sm100.cuh"
 #include "whiten.h"
@@ -376,193 +379,361 @@ __global__ void __launch_bounds__(kPcaThreads) pca_cluster(const double* __restr
     }
 }
 
-// The same power iteration with the working matrix in registers, for M up
-// to 128 * RPW (8 CTAs x 16 warps x RPW rows) and 32 * CPL columns: lane l
-// of a warp holds its RPW rows at columns l + 32 j.  Every sum is formed in
-// the order pca_cluster forms it (per-lane column sums then the XOR
-// shuffle tree for a matvec row; 32-element warp trees summed in warp order
-// for a norm or a dot product), so components, sigma and W are identical.
+// The same power iteration with the working matrix in registers: lane l of a
+// warp holds its RPW rows at columns l + 32 j (j < CPL) and the current vector
+// at the same columns.  Every sum is formed in the order pca_cluster forms it
+// (per-lane column sums, then the XOR shuffle tree), and the quotient y / sigma
+// is the correctly rounded one (div_by.cuh), so components, sigma and W have
+// the same bits.
 //
-// The matvec results are exchanged point to point instead of through a
-// cluster barrier: the warp that owns row m stores y[m] into every CTA's
-// receive buffer with st.async, whose bytes complete on the receiving CTA's
-// own mbarrier.  Every CTA also sends every CTA (itself included) an 8-byte
-// token per step, so a CTA waits for (M + CS) * 8 bytes: the tokens make
-// each step depend on every CTA having finished the previous one, also for
-// CTAs that own no rows (small M).  Step s uses buffer s & 1 (phase s >> 1
-// of its mbarrier); a CTA sends step s + 2 only after it has received all of
-// step s + 1, and every CTA sends step s + 1 after its block barrier of step
-// s, so no buffer is overwritten while it is read and no CTA's mbarrier gets
-// two phases ahead of one of its threads.  Each warp forms the norm itself
-// from the received vector, so one iteration is one matvec, one mbarrier
-// wait, the division and one block barrier.  Every wait is bounded (error
-// flag g_pca_timeout).
-constexpr int kPcaWarps = kPcaThreads / 32;
-constexpr int kPcaMaxCluster = 16;  // token slots; the register kernel runs in clusters of 8
-
+// What bounds it: the M * 11 matvec steps depend on one another, so a step's
+// latency is the time (at 384 channels one step is 147,456 FP64 FMAs, 0.15 us of
+// the FP64 pipes of 16 SMs, while DFMA takes 9 cycles, a shuffle level about 30,
+// sqrt 85 and an 8-byte exchange between two SMs 311).  A step is: read the
+// exchanged vector (CPL values per lane), norm (FMA chain, shuffle tree, sqrt),
+// v = y / sigma in registers (one reciprocal, four FMAs per value), the row
+// sums, the trees of all the warp's rows merged (each level halves the rows a
+// lane holds, so RPW rows cost about as many shuffles as one), and the
+// exchange.  Every warp forms norm and quotient itself, which costs less than
+// handing them round.
+//
+// CS = 1 (M <= 128): one CTA; rows meet in shared memory, one block barrier a
+// step.  344 us at 32 channels and 1468 us at 128 with the 8-CTA cluster that this
+// replaces; now 146 us and 1130 us.
+// CS = 16 (M > 128): sixteen CTAs of NW warps; row m belongs to CTA m % CS, so
+// every CTA owns rows.  A CTA gathers its rows in shared memory (the step's one
+// block barrier) and each warp stores them to its share of the sixteen CTAs with
+// st.async, a CTA's rows contiguous in one warp store, counted in bytes on the
+// receiver's mbarrier.  The exchange is bound by those stores: 16 x 24 rows take
+// 596 cycles that way and 880 as 8- or 16-byte stores scattered over the CTAs
+// (1130-1160 as bulk copies).  Since a CTA sends step s + 1 after all its warps
+// have read step s, having received all M rows of step s + 1 means every CTA is
+// done with step s: buffer s & 1 is free for step s + 2, and no mbarrier gets two
+// phases ahead of one of its readers.  Waits spin first (an exchange takes well
+// under a microsecond, less than a suspended wait takes to wake) and are bounded
+// (error flag g_pca_timeout).  Eight CTAs of 16 warps and 3 rows, with division
+// and vector handed round through shared memory, took 8230 us at 384 channels and
+// 3023 us at 200; this takes 4030 us and 1640 us.
 __device__ int g_pca_timeout;  // set when an exchange wait gave up (checked by the host)
 
-template <int RPW, int CPL>
-__global__ void __launch_bounds__(kPcaThreads, 1) pca_cluster_reg(const double* __restrict__ XXt, int M,
-                                                                   int num_iter, double* __restrict__ comps,
-                                                                   double* __restrict__ sigma) {
+__device__ __noinline__ double plain_quotient(double y, double b) { return y / b; }
+
+// Whether v[j] / b may use quotient_in_range for every element with 32 j < left
+// (the others are zero and stay so), as far as v decides it; called by all lanes
+// of a warp.
+template <int N>
+__device__ __forceinline__ bool quotients_in_range(const double (&v)[N], int left) {
+    bool fast = true;
+#pragma unroll
+    for (int j = 0; j < N; j++) fast &= quotient_range(v[j]) || 32 * j >= left;
+    return __all_sync(0xffffffffu, fast);
+}
+
+// v[j] = v[j] / b.  Up to two elements the ordinary division is the shorter
+// chain (one: 112 cycles against 196).
+template <int N>
+__device__ __forceinline__ void divide_by(double (&v)[N], double b, int left, bool in_range) {
+    if (N > 2) {
+        const Reciprocal c = reciprocal_of(b);
+        if (in_range && c.in_range) {
+#pragma unroll
+            for (int j = 0; j < N; j++) v[j] = quotient_in_range(v[j], b, c);
+            return;
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < N; j++)
+        if (32 * j < left) v[j] = N > 2 ? plain_quotient(v[j], b) : v[j] / b;
+}
+
+// element J0 + i (i < K) of lane `lane`'s v
+template <int J0, int K, int N>
+__device__ __forceinline__ double shfl_element(const double (&v)[N], int i, int lane) {
+    double x = v[J0];
+#pragma unroll
+    for (int k = 1; k < K; k++)
+        if (i == k) x = v[J0 + k];
+    return __shfl_sync(0xffffffffu, x, lane);
+}
+
+// out[r] = element m of the vector held as v[j] on lane l (element l + 32 j),
+// for the row slots m = r G + base, base < G
+template <int G, int R, int RPW, int N>
+__device__ __forceinline__ void row_elements_from(const double (&v)[N], int base, double (&out)[RPW]) {
+    if constexpr (R < RPW) {
+        const int m = R * G + base;
+        out[R] = shfl_element<R * G / 32, (G >= 32 ? G / 32 : 1)>(v, G >= 32 ? base >> 5 : 0, m & 31);
+        row_elements_from<G, R + 1>(v, base, out);
+    }
+}
+template <int G, int RPW, int N>
+__device__ __forceinline__ void row_elements(const double (&v)[N], int base, double (&out)[RPW]) {
+    row_elements_from<G, 0>(v, base, out);
+}
+
+__host__ __device__ constexpr int pow2_at_least(int n) { return n <= 1 ? 1 : 2 * pow2_at_least((n + 1) / 2); }
+
+template <int CS, int NW, int CPL>
+__global__ void __launch_bounds__(NW * 32, 1) pca_reg(const double* __restrict__ XXt_all, int M, int num_iter,
+                                                      double* __restrict__ comps_all,
+                                                      double* __restrict__ sigma_all) {
+    constexpr int G = CS * NW;             // rows per row slot of the whole cluster
+    constexpr int RPW = 32 * CPL / G;      // row slots of a warp
+    static_assert(RPW * G == 32 * CPL, "the rows fill the column range");
+    constexpr int RP2 = pow2_at_least(RPW);
+    static_assert(RP2 <= 32, "rows of a warp's merged tree");
+    constexpr int S = 32 / RP2;            // lanes that end up with the same row's sum
     constexpr int kMaxM = 32 * CPL;
     cg::cluster_group cluster = cg::this_cluster();
-    const int rank = (int)cluster.block_rank();
-    const int CS = (int)cluster.num_blocks();
+    const int rank = CS > 1 ? (int)cluster.block_rank() : 0;
+    const int64_t mat = blockIdx.x / CS;   // one cluster per matrix
+    const double* XXt = XXt_all + mat * M * M;
+    double* comps = comps_all + mat * M * M;
+    double* sigma = sigma_all + mat * M;
     int* err = &g_pca_timeout;
-    __shared__ double ybuf[2][kMaxM];  // matvec results, written by every CTA
-    __shared__ double vs[kMaxM];       // the normalised vector
+    // matvec results; entries beyond M stay zero.  CS > 1: row m at (m % CS) * RS
+    // + m / CS, so that a CTA's rows are contiguous; RS odd keeps the strided
+    // reads free of bank conflicts.
+    constexpr int R = NW * RPW;  // rows of a CTA
+    constexpr int RS = R | 1;
+    static_assert(CS == 1 || R <= 32, "a CTA's rows in one warp store");
+    constexpr int kYLen = CS > 1 ? CS * RS : kMaxM;
+    __shared__ double ybuf[2][kYLen];
+    __shared__ double stage[2][CS > 1 ? R : 1];  // CS > 1: this CTA's rows on their way out
     __shared__ double vinit[kMaxM];
-    __shared__ double red[32];
-    __shared__ __align__(8) uint64_t ybar[2];  // bytes of ybuf[b] received in the current step
-    __shared__ __align__(8) uint64_t tok[2][kPcaMaxCluster];  // one token per sending CTA and step
+    __shared__ __align__(8) uint64_t ybar[2];  // CS > 1: bytes of ybuf[b] received in the current step
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    const int row0 = (rank * kPcaWarps + w) * RPW;
-    const bool has_rows = row0 < M;
-    const uint32_t step_bytes = (uint32_t)(M + CS) * 8u;
+    const int base = w * CS + rank;  // row of slot 0
+    const uint32_t step_bytes = (uint32_t)M * 8u;
 
     double A[RPW][CPL];
 #pragma unroll
     for (int r = 0; r < RPW; r++)
 #pragma unroll
         for (int j = 0; j < CPL; j++) {
-            const int m = row0 + r, n = l + 32 * j;
+            const int m = r * G + base, n = l + 32 * j;
             A[r][j] = (m < M && n < M) ? XXt[(size_t)m + (size_t)M * n] : 0.0;
         }
-    if (threadIdx.x == 0) {
+    for (int n = threadIdx.x; n < 2 * kYLen; n += NW * 32) (&ybuf[0][0])[n] = 0.0;
+    if (CS > 1 && threadIdx.x == 0) {
         tc::mbar_init(&ybar[0], 1);
         tc::mbar_init(&ybar[1], 1);
         tc::fence_mbar_init();
     }
-    // start vector sin(i+1), normalised (pca.cpp:546-549, 457-466)
-    for (int n = threadIdx.x; n < M; n += blockDim.x) vinit[n] = sin((double)(n + 1));
-    __syncthreads();
+    double v[CPL];
+    // start vector sin(i+1), normalised (pca.cpp:546-549, 457-466); squares
+    // summed per 32 elements (tree), then chunk after chunk
     {
-        double part = 0.0;
-        for (int n = threadIdx.x; n < M; n += blockDim.x) part += vinit[n] * vinit[n];
-        const double nrm = sqrt(block_sum(part, red));
-        __syncthreads();
-        if (nrm != 0.0)
-            for (int n = threadIdx.x; n < M; n += blockDim.x) vinit[n] = vinit[n] / nrm;
+        double nrm2 = 0.0;
+#pragma unroll
+        for (int j = 0; j < CPL; j++) {
+            const int n = l + 32 * j;
+            v[j] = n < M ? sin((double)(n + 1)) : 0.0;
+            double p = __dmul_rn(v[j], v[j]);
+            for (int o = 16; o > 0; o >>= 1) p += __shfl_xor_sync(0xffffffffu, p, o);
+            nrm2 += p;
+        }
+        const double nrm = sqrt(nrm2);
+#pragma unroll
+        for (int j = 0; j < CPL; j++) {
+            if (nrm != 0.0 && l + 32 * j < M) v[j] = v[j] / nrm;
+            if (w == 0) vinit[l + 32 * j] = v[j];
+        }
     }
-    if (threadIdx.x == 0) {
+    if (CS > 1 && threadIdx.x == 0) {
         tc::mbar_expect_tx(&ybar[0], step_bytes);  // steps 0 and 1
         tc::mbar_expect_tx(&ybar[1], step_bytes);
     }
     // every CTA's barriers are initialised and armed before any store reaches them
-    cluster.sync();
-    // lane l < CS sends to CTA l: the cluster addresses of its buffers and barriers
-    const uint32_t rbuf = l < CS ? tc::mapa_shared(tc::smem_u32(&ybuf[0][0]), (uint32_t)l) : 0u;
-    const uint32_t rbar = l < CS ? tc::mapa_shared(tc::smem_u32(&ybar[0]), (uint32_t)l) : 0u;
-    const uint32_t rtok = l < CS ? tc::mapa_shared(tc::smem_u32(&tok[0][0]), (uint32_t)l) : 0u;
+    if (CS > 1)
+        cluster.sync();
+    else
+        __syncthreads();
 
-    // y = A v for this warp's rows, stored into every CTA's ybuf[step & 1];
-    // then the wait for the whole vector of the step
-    auto matvec = [&](const double* v, int64_t step) -> bool {
-        const int b = (int)(step & 1);
-        if (w == 0 && l < CS)
-            tc::st_async_b64(rtok + (uint32_t)((b * kPcaMaxCluster + rank) * 8), 0ull, rbar + (uint32_t)(b * 8));
-        if (has_rows) {
-            double s[RPW];
+    // the row whose sum this lane holds after the merged tree: bit 4 of the lane
+    // selects the upper half of the slots, bit 3 the upper half of those, ...
+    int slot = 0;
 #pragma unroll
-            for (int r = 0; r < RPW; r++) s[r] = 0.0;
+    for (int o = 16, h = RP2 / 2; h > 0; o >>= 1, h >>= 1) slot += (l & o) ? h : 0;
+    const bool holds = slot < RPW && slot * G + base < M && l % S == 0;
+    // CS > 1: warp w stores the CTA's rows to the CTAs w + NW i, lane q row q CS + rank
+    constexpr int kSends = CS > 1 ? CS / NW : 1;
+    uint32_t rbuf[kSends], rbar[kSends];
+    const bool sends = l < R && l * CS + rank < M;
+    if (CS > 1) {
 #pragma unroll
-            for (int j = 0; j < CPL; j++) {
-                const int n = l + 32 * j;
-                if (n < M) {
-                    const double vn = v[n];
+        for (int i = 0; i < kSends; i++) {
+            const uint32_t d = (uint32_t)(w + NW * i);
+            rbuf[i] = tc::mapa_shared(tc::smem_u32(&ybuf[0][0]), d) + (uint32_t)(rank * RS + l) * 8u;
+            rbar[i] = tc::mapa_shared(tc::smem_u32(&ybar[0]), d);
+        }
+    }
+    // where this lane finds element l + 32 j of a vector in ybuf
+    const int y0 = CS > 1 ? (l % CS) * RS + l / CS : l;
+    constexpr int kYStep = CS > 1 ? 32 / CS : 32;
+
+    // ybuf[step & 1] = A v in every CTA; returns once it is complete
+    auto matvec = [&](int step) -> bool {
+        const int b = step & 1;
+        double s[RP2];
 #pragma unroll
-                    for (int r = 0; r < RPW; r++) s[r] += A[r][j] * vn;
-                }
-            }
+        for (int r = 0; r < RP2; r++) s[r] = 0.0;
 #pragma unroll
-            for (int r = 0; r < RPW; r++) {
-                for (int o = 16; o > 0; o >>= 1) s[r] += __shfl_xor_sync(0xffffffffu, s[r], o);
-                const int m = row0 + r;
-                if (m < M && l < CS)
-                    tc::st_async_b64(rbuf + (uint32_t)((b * kMaxM + m) * 8), (uint64_t)__double_as_longlong(s[r]),
-                                     rbar + (uint32_t)(b * 8));
+        for (int j = 0; j < CPL; j++)
+#pragma unroll
+            for (int r = 0; r < RPW; r++) s[r] = __fma_rn(A[r][j], v[j], s[r]);
+        int o = 16;
+#pragma unroll
+        for (int h = RP2 / 2; h > 0; h >>= 1, o >>= 1) {
+            const bool up = (l & o) != 0;
+#pragma unroll
+            for (int i = 0; i < h; i++) {
+                const double keep = up ? s[i + h] : s[i], give = up ? s[i] : s[i + h];
+                s[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
             }
         }
-        const bool ok = tc::mbar_wait_cluster(&ybar[b], (uint32_t)((step >> 1) & 1), err);
+#pragma unroll
+        for (int q = S / 2; q > 0; q >>= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], q);
+        if (CS == 1) {
+            if (holds) ybuf[b][slot * G + base] = s[0];
+            __syncthreads();
+            return true;
+        }
+        if (holds) stage[b][slot * NW + w] = s[0];
+        __syncthreads();
+        if (sends) {
+            const uint64_t x = (uint64_t)__double_as_longlong(stage[b][l]);
+#pragma unroll
+            for (int i = 0; i < kSends; i++)
+                tc::st_async_b64(rbuf[i] + (uint32_t)(b * kYLen * 8), x, rbar[i] + (uint32_t)(b * 8));
+        }
+        const bool ok = __all_sync(0xffffffffu, tc::mbar_wait_cluster_spin(&ybar[b], (uint32_t)((step >> 1) & 1), err));
         // re-arm for step + 2: its stores arrive only after this CTA has sent step + 1
         if (ok && threadIdx.x == 0) tc::mbar_expect_tx(&ybar[b], step_bytes);
         return ok;
     };
 
-    int64_t step = 0;  // matvec count (same sequence in every CTA)
+    int step = 0;  // matvec count, at most 512 * 11 (the same sequence in every warp)
     bool ok = true;
     for (int k = 0; k < M && ok; k++) {
-        const double* v = vinit;
+#pragma unroll
+        for (int j = 0; j < CPL; j++) v[j] = vinit[l + 32 * j];
         double sig = 0.0;
-        for (int it = 0; it < num_iter; it++) {
-            const bool got = matvec(v, step);
-            const double* y = ybuf[step & 1];
-            if (got) {
-                sig = sqrt(warp_ordered_sum(M, [&](int n) { return y[n] * y[n]; }));
-                for (int n = threadIdx.x; n < M; n += blockDim.x) vs[n] = sig != 0.0 ? y[n] / sig : y[n];
-            }
-            ok = __syncthreads_and(got) != 0;
+        for (int it = 0; it < num_iter && ok; it++) {
+            ok = matvec(step);
             if (!ok) break;
-            v = vs;
+            const double* y = ybuf[step & 1];
             step++;
+            double t = 0.0;
+#pragma unroll
+            for (int j = 0; j < CPL; j++) {
+                v[j] = y[y0 + kYStep * j];
+                t = __fma_rn(v[j], v[j], t);
+            }
+            const bool in_range = CPL > 2 && quotients_in_range<CPL>(v, M - l);
+            for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+            sig = sqrt(t);
+            if (sig != 0.0) divide_by<CPL>(v, sig, M - l, in_range);
         }
         if (!ok) break;
-        if (rank == 0) {
-            for (int n = threadIdx.x; n < M; n += blockDim.x) comps[(size_t)n + (size_t)M * k] = v[n];
-            if (threadIdx.x == 0) sigma[k] = sig;
+        if (rank == 0 && w == 0) {
+#pragma unroll
+            for (int j = 0; j < CPL; j++)
+                if (l + 32 * j < M) comps[(size_t)(l + 32 * j) + (size_t)M * k] = v[j];
+            if (l == 0) sigma[k] = sig;
         }
         // deflation: X <- X - v u' - u v' + (v'u) v v',  u = X v
-        const bool got = matvec(v, step);
+        ok = matvec(step);
+        if (!ok) break;
         const double* u = ybuf[step & 1];
         step++;
-        if (got && has_rows) {
-            const double alpha = warp_ordered_sum(M, [&](int n) { return v[n] * u[n]; });
+        double uj[CPL];
+        double alpha = 0.0;
 #pragma unroll
-            for (int r = 0; r < RPW; r++) {
-                const int m = row0 + r;
-                if (m >= M) continue;
-                const double vm = v[m], um = u[m];
+        for (int j = 0; j < CPL; j++) {
+            uj[j] = u[y0 + kYStep * j];
+            alpha = __fma_rn(v[j], uj[j], alpha);
+        }
+        for (int o = 16; o > 0; o >>= 1) alpha += __shfl_xor_sync(0xffffffffu, alpha, o);
+        double vm_of[RPW];
+        row_elements<G, RPW>(v, base, vm_of);
 #pragma unroll
-                for (int j = 0; j < CPL; j++) {
-                    const int n = l + 32 * j;
-                    if (n < M) {
-                        const double sdef = __dadd_rn(__dmul_rn(vm, u[n]), __dmul_rn(um, v[n]));
-                        const double x = __dsub_rn(A[r][j], sdef);
-                        A[r][j] = __dadd_rn(x, __dmul_rn(alpha, __dmul_rn(vm, v[n])));
-                    }
+        for (int r = 0; r < RPW; r++) {
+            const double vm = vm_of[r], um = u[CS > 1 ? rank * RS + r * NW + w : r * G + base];
+#pragma unroll
+            for (int j = 0; j < CPL; j++) {
+                if (l + 32 * j < M) {
+                    const double sdef = __dadd_rn(__dmul_rn(vm, uj[j]), __dmul_rn(um, v[j]));
+                    const double x = __dsub_rn(A[r][j], sdef);
+                    A[r][j] = __dadd_rn(x, __dmul_rn(alpha, __dmul_rn(vm, v[j])));
                 }
             }
         }
-        // vs and this buffer are read above; the next component rewrites vs
-        // after its first wait and the buffer two steps later
-        ok = __syncthreads_and(got) != 0;
     }
     // no CTA leaves while a peer may still store into its shared memory
-    cluster.sync();
+    if (CS > 1) cluster.sync();
 }
 
 // W = (C D) C^T, D = diag(1/sqrt(sigma)) (0 where sigma == 0), in the
 // reference's order: tmp(m,l) = C(m,l) d_l (mult_AB with a diagonal,
 // pca.cpp:220-243), W(m,n) = sum_l tmp(m,l) C(n,l) (mult_ABtrans, :319-342).
-__global__ void w_assemble(const double* __restrict__ C, const double* __restrict__ sigma, int M,
-                           double* __restrict__ W) {
-    extern __shared__ double dsh[];
-    for (int l = threadIdx.x; l < M; l += blockDim.x) {
-        const double s = sigma[l];
-        dsh[l] = (s != 0.0) ? 1.0 / sqrt(s) : 0.0;
+// A 32 x 32 tile of W per block, the l range staged through shared memory 32 at a
+// time (tmp formed there once per tile), 2 x 2 sums per thread.  The sums are
+// serial in l: one thread per element reading C from L2 spent its time on the
+// loads (115 us at 384 channels; now 34 us).  blockIdx.z: the matrix of a batch.
+constexpr int kWT = 32;
+__global__ void __launch_bounds__(256) w_assemble(const double* __restrict__ C_all,
+                                                  const double* __restrict__ sigma_all, int M,
+                                                  double* __restrict__ W_all) {
+    __shared__ double tmp[kWT][kWT], cn[kWT][kWT];  // [l][m], [l][n]
+    __shared__ double dl[2][kWT];                   // d of the l tile in flight
+    const double* C = C_all + (size_t)blockIdx.z * M * M;
+    const double* sigma = sigma_all + (size_t)blockIdx.z * M;
+    double* W = W_all + (size_t)blockIdx.z * M * M;
+    const int m0 = blockIdx.x * kWT, n0 = blockIdx.y * kWT;
+    const int x = threadIdx.x & 31, y = threadIdx.x >> 5;  // staging: element x of rows y + 8 i
+    const int mi = threadIdx.x & 15, ni = threadIdx.x >> 4;  // sums: m0 + mi + 16 a, n0 + ni + 16 b
+    double a[4], c[4];
+    auto fetch = [&](int l0) {
+        if (y == 0) {
+            const double s = l0 + x < M ? sigma[l0 + x] : 0.0;
+            dl[(l0 / kWT) & 1][x] = (s != 0.0) ? 1.0 / sqrt(s) : 0.0;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int l = l0 + y + 8 * i;
+            a[i] = (l < M && m0 + x < M) ? C[(size_t)(m0 + x) + (size_t)M * l] : 0.0;
+            c[i] = (l < M && n0 + x < M) ? C[(size_t)(n0 + x) + (size_t)M * l] : 0.0;
+        }
+    };
+    double acc[2][2] = {};
+    fetch(0);
+    for (int l0 = 0; l0 < M; l0 += kWT) {
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            tmp[y + 8 * i][x] = __dmul_rn(a[i], dl[(l0 / kWT) & 1][y + 8 * i]);
+            cn[y + 8 * i][x] = c[i];
+        }
+        __syncthreads();
+        if (l0 + kWT < M) fetch(l0 + kWT);
+        const int nl = min(kWT, M - l0);
+#pragma unroll 8
+        for (int l = 0; l < nl; l++) {
+            const double t0 = tmp[l][mi], t1 = tmp[l][mi + 16], c0 = cn[l][ni], c1 = cn[l][ni + 16];
+            acc[0][0] = __dadd_rn(acc[0][0], __dmul_rn(t0, c0));
+            acc[0][1] = __dadd_rn(acc[0][1], __dmul_rn(t0, c1));
+            acc[1][0] = __dadd_rn(acc[1][0], __dmul_rn(t1, c0));
+            acc[1][1] = __dadd_rn(acc[1][1], __dmul_rn(t1, c1));
+        }
     }
-    __syncthreads();
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    const int n = blockIdx.y;
-    if (m >= M) return;
-    double acc = 0.0;
-    for (int l = 0; l < M; l++) {
-        const double tmp = __dmul_rn(C[(size_t)m + (size_t)M * l], dsh[l]);
-        acc = __dadd_rn(acc, __dmul_rn(tmp, C[(size_t)n + (size_t)M * l]));
-    }
-    W[(size_t)m + (size_t)M * n] = acc;
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const int m = m0 + mi + 16 * i, n = n0 + ni + 16 * j;
+            if (m < M && n < M) W[(size_t)m + (size_t)M * n] = acc[i][j];
+        }
 }
 
 // ------------------------------------------------------------ apply
@@ -864,6 +1035,57 @@ void covariance_device_noalloc(const float* X, int64_t M, int64_t N, double* XXt
 // pca_cluster launch: rows in shared memory across 8 or 16 CTAs, else in global memory.
 void pca_launch_smem(const double* XXt, int64_t M, double* comps, double* sigma, cudaStream_t stream);
 
+namespace {
+
+// pca_reg for `count` matrices, one cluster each; false when the device cannot
+// hold a cluster of that size.
+template <int CS, int NW, int CPL>
+bool launch_pca_reg(const double* XXt, int64_t M, int count, double* comps, double* sigma, cudaStream_t stream) {
+    auto kern = pca_reg<CS, NW, CPL>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(CS * count), 1, 1);
+    cfg.blockDim = dim3(NW * 32, 1, 1);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = CS;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (CS > 8) {
+        MS3_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            clusters = 0;
+        }
+        if (clusters < 1) return false;
+    }
+    MS3_CUDA(cudaLaunchKernelEx(&cfg, kern, XXt, (int)M, 10, comps, sigma));
+    MS3_LAUNCH_CHECK();
+    return true;
+}
+
+// Up to 128 channels the matrix fits one CTA's registers (128 KB at most) and
+// an exchange through shared memory costs less than one between SMs (128 channels:
+// 0.80 us a step in one CTA, 1.04 in a cluster of eight); beyond, 16 CTAs hold it.
+// The smallest instance whose column range covers M.
+bool pca_registers(const double* XXt, int64_t M, int count, double* comps, double* sigma, cudaStream_t stream) {
+    if (M <= 32) return launch_pca_reg<1, 4, 1>(XXt, M, count, comps, sigma, stream);
+    if (M <= 64) return launch_pca_reg<1, 8, 2>(XXt, M, count, comps, sigma, stream);
+    if (M <= 96) return launch_pca_reg<1, 8, 3>(XXt, M, count, comps, sigma, stream);
+    if (M <= 128) return launch_pca_reg<1, 8, 4>(XXt, M, count, comps, sigma, stream);
+    if (M <= 192) return launch_pca_reg<16, 4, 6>(XXt, M, count, comps, sigma, stream);
+    if (M <= 256) return launch_pca_reg<16, 4, 8>(XXt, M, count, comps, sigma, stream);
+    if (M <= 320) return launch_pca_reg<16, 4, 10>(XXt, M, count, comps, sigma, stream);
+    if (M <= 384) return launch_pca_reg<16, 4, 12>(XXt, M, count, comps, sigma, stream);
+    if (M <= 512) return launch_pca_reg<16, 8, 16>(XXt, M, count, comps, sigma, stream);
+    return false;
+}
+
+}  // namespace
+
 void whitening_matrix_device(const double* XXt, int64_t M, double* W, double* comps, double* sigma,
                              cudaStream_t stream) {
     if (M <= 0) return;
@@ -872,34 +1094,15 @@ void whitening_matrix_device(const double* XXt, int64_t M, double* W, double* co
     if (!comps) { cbuf.alloc(sizeof(double) * (size_t)(M * M), stream); comps = cbuf.as<double>(); }
     if (!sigma) { sbuf.alloc(sizeof(double) * (size_t)M, stream); sigma = sbuf.as<double>(); }
 
-    // registers hold the working matrix up to 384 channels (MS3GPU_PCA_KERNEL=smem
+    // registers hold the working matrix up to 512 channels (MS3GPU_PCA_KERNEL=smem
     // selects the shared-memory kernel, which gives the same values)
     const char* pk = std::getenv("MS3GPU_PCA_KERNEL");
     const bool force_smem = pk && std::string(pk) == "smem";
     const char* force_global0 = std::getenv("MS3GPU_PCA_ROWS_GLOBAL");
-    if (!force_smem && !(force_global0 && force_global0[0] == '1') && M <= 384) {
-        auto kern = M <= 128 ? pca_cluster_reg<1, 4> : (M <= 256 ? pca_cluster_reg<2, 8> : pca_cluster_reg<3, 12>);
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(8, 1, 1);
-        cfg.blockDim = dim3(kPcaThreads, 1, 1);
-        cfg.dynamicSmemBytes = 0;
-        cfg.stream = stream;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 8;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        MS3_CUDA(cudaLaunchKernelEx(&cfg, kern, XXt, (int)M, 10, comps, sigma));
-        MS3_LAUNCH_CHECK();
-    } else {
-        pca_launch_smem(XXt, M, comps, sigma, stream);
-    }
-    const size_t wsm = sizeof(double) * (size_t)M;
-    if (wsm > 48 * 1024)
-        MS3_CUDA(cudaFuncSetAttribute(w_assemble, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wsm));
-    w_assemble<<<dim3((unsigned)ceil_div(M, 128), (unsigned)M), 128, wsm, stream>>>(comps, sigma, (int)M, W);
+    const bool registers = !force_smem && !(force_global0 && force_global0[0] == '1');
+    if (!registers || !pca_registers(XXt, M, 1, comps, sigma, stream)) pca_launch_smem(XXt, M, comps, sigma, stream);
+    const unsigned wt = (unsigned)ceil_div(M, kWT);
+    w_assemble<<<dim3(wt, wt), 256, 0, stream>>>(comps, sigma, (int)M, W);
     MS3_LAUNCH_CHECK();
 }
 
