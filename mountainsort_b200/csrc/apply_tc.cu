@@ -104,10 +104,10 @@ __device__ __forceinline__ uint32_t x_lo_tf32(uint32_t xb) {
 // Stores 32 consecutive output channels of one timepoint, already rounded
 // to 1e-4; int16 output is scaled by the quantization unit as the reference
 // does ((int)(x / q + 0.5) truncated to 16 bits).
-__device__ __forceinline__ void store_row32(const float (&y)[32], int64_t t, int64_t nbase, int64_t M, double qunit,
-                                            void* __restrict__ out) {
+__device__ __forceinline__ void store_row32(const float (&y)[32], int64_t t, int64_t nbase, int64_t M, int64_t ld,
+                                            double qunit, void* __restrict__ out) {
     if (qunit > 0) {
-        int16_t* o16 = static_cast<int16_t*>(out) + t * M;
+        int16_t* o16 = static_cast<int16_t*>(out) + t * ld;
 #pragma unroll
         for (int j = 0; j < 32; j++) {
             if (nbase + j >= M) break;
@@ -116,7 +116,7 @@ __device__ __forceinline__ void store_row32(const float (&y)[32], int64_t t, int
         }
         return;
     }
-    float* of = static_cast<float*>(out) + t * M + nbase;
+    float* of = static_cast<float*>(out) + t * ld + nbase;
     if (nbase + 32 <= M && ((reinterpret_cast<uintptr_t>(of) & 15) == 0)) {
 #pragma unroll
         for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(of + j) = make_float4(y[j], y[j + 1], y[j + 2], y[j + 3]);
@@ -134,7 +134,7 @@ __device__ __forceinline__ void store_row32(const float (&y)[32], int64_t t, int
 // 32 x 32 block (full 128-byte lines), int16 output directly.
 __device__ __forceinline__ void emit_row32(float (&y)[32], int lane, uint8_t* staging_warp, int& sbuf,
                                            const CUtensorMap* tmOut, int out_tma, int64_t t, int64_t trow0, int n,
-                                           int64_t M, int64_t N, double qunit, int round_1e4,
+                                           int64_t M, int64_t N, int64_t ld, double qunit, int round_1e4,
                                            void* __restrict__ out) {
     // a float block that starts beyond the last row or column would be clipped
     // whole: nothing is staged or stored, and the staging ring does not turn
@@ -158,7 +158,7 @@ __device__ __forceinline__ void emit_row32(float (&y)[32], int lane, uint8_t* st
         }
         sbuf ^= 1;
     } else if (t < N) {
-        store_row32(y, t, n, M, qunit, out);
+        store_row32(y, t, n, M, ld, qunit, out);
     }
 }
 
@@ -182,7 +182,7 @@ template <int BN, bool DRAIN>
 __global__ void __launch_bounds__(TcCfg<BN, DRAIN>::kThreads, 1)
     apply_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmWhi,
                     const __grid_constant__ CUtensorMap tmWlo, const __grid_constant__ CUtensorMap tmOut, int out_tma,
-                    int64_t M, int64_t N, int ncb, int64_t ntiles, double qunit, int round_1e4,
+                    int64_t M, int64_t N, int64_t ld, int ncb, int64_t ntiles, double qunit, int round_1e4,
                     void* __restrict__ out, int* __restrict__ err) {
     using C = TcCfg<BN, DRAIN>;
     constexpr int S = C::kStages;
@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(TcCfg<BN, DRAIN>::kThreads, 1)
                     float y[32];
 #pragma unroll
                     for (int j = 0; j < 32; j++) y[j] = __uint_as_float(r[j]);
-                    emit_row32(y, lane, stg, sbuf, &tmOut, out_tma, t, t0 + q * 32, n0 + c0, M, N, qunit, round_1e4, out);
+                    emit_row32(y, lane, stg, sbuf, &tmOut, out_tma, t, t0 + q * 32, n0 + c0, M, N, ld, qunit, round_1e4, out);
                 }
                 tc::tc_fence_before();
                 tc::mbar_arrive(&acc_free[tp]);
@@ -425,7 +425,7 @@ __global__ void __launch_bounds__(TcCfg<BN, DRAIN>::kThreads, 1)
                 float y[32];
 #pragma unroll
                 for (int j = 0; j < 32; j++) y[j] = __uint_as_float(r[j]);
-                emit_row32(y, lane, stg, sbuf, &tmOut, out_tma, t, t0 + q * 32, n0 + c0, M, N, qunit, round_1e4, out);
+                emit_row32(y, lane, stg, sbuf, &tmOut, out_tma, t, t0 + q * 32, n0 + c0, M, N, ld, qunit, round_1e4, out);
             }
         }
         if (out_tma && lane == 0) tc::bulk_wait_group<0>();  // stores complete before the CTA exits
@@ -462,11 +462,12 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
     return fn;
 }
 
-// Row-major [rows][cols] float32 matrix, tiles of box_rows x 32 columns, 128-byte swizzle.
-CUtensorMap make_map(const void* base, uint64_t cols, uint64_t rows, uint32_t box_rows) {
+// Row-major [rows][cols] float32 matrix with `ld` elements between rows, tiles of
+// box_rows x 32 columns, 128-byte swizzle.
+CUtensorMap make_map(const void* base, uint64_t cols, uint64_t rows, uint64_t ld, uint32_t box_rows) {
     CUtensorMap m;
     const cuuint64_t dims[2] = {cols, rows};
-    const cuuint64_t strides[1] = {cols * sizeof(float)};
+    const cuuint64_t strides[1] = {ld * sizeof(float)};
     const cuuint32_t box[2] = {(cuuint32_t)kKB, box_rows};
     const cuuint32_t es[2] = {1, 1};
     const CUresult r = encode_fn()(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box,
@@ -477,24 +478,24 @@ CUtensorMap make_map(const void* base, uint64_t cols, uint64_t rows, uint32_t bo
 }
 
 template <int BN, bool DRAIN>
-void launch_apply_tc(const float* X, int64_t M, int64_t N, const float* whi, const float* wlo, double qunit,
+void launch_apply_tc(const float* X, int64_t M, int64_t N, int64_t ld, const float* whi, const float* wlo, double qunit,
                      int round_1e4, void* out, int* err, cudaStream_t stream) {
     using C = TcCfg<BN, DRAIN>;
     MS3_CUDA(cudaFuncSetAttribute(apply_tc_kernel<BN, DRAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)C::kSmemBytes));
-    const CUtensorMap mx = make_map(X, (uint64_t)M, (uint64_t)N, kTM);
-    const CUtensorMap mh = make_map(whi, (uint64_t)M, (uint64_t)M, BN);
-    const CUtensorMap ml = make_map(wlo, (uint64_t)M, (uint64_t)M, BN);
+    const CUtensorMap mx = make_map(X, (uint64_t)M, (uint64_t)N, (uint64_t)ld, kTM);
+    const CUtensorMap mh = make_map(whi, (uint64_t)M, (uint64_t)M, (uint64_t)M, BN);
+    const CUtensorMap ml = make_map(wlo, (uint64_t)M, (uint64_t)M, (uint64_t)M, BN);
     // float output goes out through TMA stores of 32 x 32 blocks
     const int out_tma = (qunit <= 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0) ? 1 : 0;
-    const CUtensorMap mo = out_tma ? make_map(out, (uint64_t)M, (uint64_t)N, 32) : mx;
+    const CUtensorMap mo = out_tma ? make_map(out, (uint64_t)M, (uint64_t)N, (uint64_t)ld, 32) : mx;
     const int ncb = (int)ceil_div(M, BN);
     const int64_t ntiles = ceil_div(N, kTM) * ncb;
     int dev = 0, nsm = 0;
     MS3_CUDA(cudaGetDevice(&dev));
     MS3_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     const int64_t grid = std::min<int64_t>(ntiles, nsm);  // one persistent CTA per SM
-    apply_tc_kernel<BN, DRAIN><<<(unsigned)grid, C::kThreads, C::kSmemBytes, stream>>>(mx, mh, ml, mo, out_tma, M, N, ncb,
+    apply_tc_kernel<BN, DRAIN><<<(unsigned)grid, C::kThreads, C::kSmemBytes, stream>>>(mx, mh, ml, mo, out_tma, M, N, ld, ncb,
                                                                                      ntiles, qunit, round_1e4,
                                                                                      out, err);
     MS3_LAUNCH_CHECK();
@@ -502,7 +503,8 @@ void launch_apply_tc(const float* X, int64_t M, int64_t N, const float* whi, con
 
 }  // namespace
 
-bool apply_tc_supported(const float* X, int64_t M, int64_t N, const void* out) {
+bool apply_tc_supported(const float* X, int64_t M, int64_t N, const void* out, int64_t ld) {
+    if (ld % 4 != 0) return false;
     if (M < 4 || M % 4 != 0 || M > 65536 || N < 1) return false;  // TMA: 16-byte row strides
     if ((reinterpret_cast<uintptr_t>(X) & 15) != 0) return false;
     (void)out;
@@ -510,7 +512,7 @@ bool apply_tc_supported(const float* X, int64_t M, int64_t N, const void* out) {
 }
 
 void apply_whitening_tc(const float* X, int64_t M, int64_t N, const double* W, double quantization_unit,
-                        bool drain, void* out, cudaStream_t stream, int* ext_err, bool round_1e4) {
+                        bool drain, void* out, cudaStream_t stream, int* ext_err, bool round_1e4, int64_t ld) {
     DevBuf wbuf(sizeof(float) * (size_t)(2 * M * M) + 256, stream);
     float* whi = wbuf.as<float>();
     float* wlo = whi + M * M;
@@ -519,9 +521,9 @@ void apply_whitening_tc(const float* X, int64_t M, int64_t N, const double* W, d
     w_split_tf32<<<(unsigned)ceil_div(M * M, 256), 256, 0, stream>>>(W, M * M, whi, wlo);
     MS3_LAUNCH_CHECK();
     if (drain)
-        launch_apply_tc<128, true>(X, M, N, whi, wlo, quantization_unit, round_1e4 ? 1 : 0, out, err, stream);
+        launch_apply_tc<128, true>(X, M, N, ld, whi, wlo, quantization_unit, round_1e4 ? 1 : 0, out, err, stream);
     else
-        launch_apply_tc<128, false>(X, M, N, whi, wlo, quantization_unit, round_1e4 ? 1 : 0, out, err, stream);
+        launch_apply_tc<128, false>(X, M, N, ld, whi, wlo, quantization_unit, round_1e4 ? 1 : 0, out, err, stream);
     if (ext_err) return;  // the caller checks the flag once for many calls
     int herr = 0;
     MS3_CUDA(cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, stream));

@@ -731,20 +731,61 @@ int ms3gpu_whiten_blocks(const float* timeseries, int64_t M, int64_t N, const in
         MS3_CUDA(cudaMemcpyAsync(chmap.get(), ch0.data(), sizeof(int32_t) * (size_t)M, cudaMemcpyHostToDevice, s));
         DevBuf err(sizeof(int), s);
         MS3_CUDA(cudaMemsetAsync(err.get(), 0, sizeof(int), s));
-        int64_t off = 0;
+        // The matrices of all blocks first, then the applies: a power iteration is a
+        // chain of dependent steps on 1 or 16 SMs, so those of neighbouring blocks of
+        // one size run side by side (4 blocks of 384 channels: 4.0 ms instead of 16.1).
+        // A block of adjacent channels at 16-byte boundaries is read and written in
+        // place in the recording's rows (unless those are also the output's); other blocks go through a gathered copy, made
+        // again for the apply so that one block's copies are held at a time.
+        const float* X = static_cast<const float*>(in.ptr);
+        std::vector<int64_t> off((size_t)n_blocks + 1, 0), moff((size_t)n_blocks + 1, 0);
+        for (int32_t k = 0; k < n_blocks; k++) {
+            off[(size_t)k + 1] = off[(size_t)k] + block_sizes[k];
+            moff[(size_t)k + 1] = moff[(size_t)k] + (int64_t)block_sizes[k] * block_sizes[k];
+        }
+        const uintptr_t x0 = reinterpret_cast<uintptr_t>(X), o0 = reinterpret_cast<uintptr_t>(out.ptr);
+        const bool apart = x0 + in_bytes <= o0 || o0 + esz * (size_t)(M * N) <= x0;  // X and out share no byte
+        auto in_place = [&](int32_t k) {
+            const int64_t Mb = block_sizes[k], o = off[(size_t)k];
+            if (!apart) return false;
+            for (int64_t j = 1; j < Mb; j++)
+                if (ch0[(size_t)(o + j)] != ch0[(size_t)o] + j) return false;
+            return M % 4 == 0 && Mb % 4 == 0 && ch0[(size_t)o] % 4 == 0 && x0 % 16 == 0;
+        };
+        auto gather = [&](int32_t k, DevBuf& xb) {
+            const int64_t Mb = block_sizes[k];
+            xb.alloc(sizeof(float) * (size_t)(Mb * N), s);
+            gather_channels_device(X, M, N, chmap.as<int32_t>() + off[(size_t)k], Mb, xb.as<float>(), s);
+            return xb.as<float>();
+        };
+        DevBuf mats(sizeof(double) * (size_t)(2 * moff[(size_t)n_blocks]), s);
+        double* XXt = mats.as<double>();
+        double* W = XXt + moff[(size_t)n_blocks];
+        DevBuf only;  // a single block's copy serves both passes
         for (int32_t k = 0; k < n_blocks; k++) {
             const int64_t Mb = block_sizes[k];
-            const int32_t* chk = chmap.as<int32_t>() + off;
-            DevBuf xb(sizeof(float) * (size_t)(Mb * N), s), yb(esz * (size_t)(Mb * N), s);
-            DevBuf mats(sizeof(double) * (size_t)(2 * Mb * Mb), s);
-            gather_channels_device(static_cast<const float*>(in.ptr), M, N, chk, Mb, xb.as<float>(), s);
-            double* XXt = mats.as<double>();
-            double* W = XXt + Mb * Mb;
-            covariance_device(xb.as<float>(), Mb, N, XXt, s);
-            whitening_matrix_device(XXt, Mb, W, nullptr, nullptr, s);
-            apply_whitening_device(xb.as<float>(), Mb, N, W, q, mixed, yb.get(), s, err.as<int>());
-            scatter_channels_device(yb.get(), Mb, N, chk, M, out.ptr, esz, s);
-            off += Mb;
+            if (in_place(k)) {
+                covariance_device(X + ch0[(size_t)off[(size_t)k]], Mb, N, XXt + moff[(size_t)k], s, M);
+            } else {
+                DevBuf mine;
+                covariance_device(gather(k, n_blocks == 1 ? only : mine), Mb, N, XXt + moff[(size_t)k], s);
+            }
+        }
+        for (int32_t k = 0, e; k < n_blocks; k = e) {
+            for (e = k + 1; e < n_blocks && block_sizes[e] == block_sizes[k]; e++) {}
+            whitening_matrix_device(XXt + moff[(size_t)k], block_sizes[k], W + moff[(size_t)k], nullptr, nullptr, s, e - k);
+        }
+        for (int32_t k = 0; k < n_blocks; k++) {
+            const int64_t Mb = block_sizes[k], c0 = ch0[(size_t)off[(size_t)k]];
+            if (in_place(k)) {
+                apply_whitening_device(X + c0, Mb, N, W + moff[(size_t)k], q, mixed,
+                                       static_cast<char*>(out.ptr) + esz * (size_t)c0, s, err.as<int>(), true, M);
+                continue;
+            }
+            DevBuf mine, yb(esz * (size_t)(Mb * N), s);
+            const float* xb = only.get() ? only.as<float>() : gather(k, mine);
+            apply_whitening_device(xb, Mb, N, W + moff[(size_t)k], q, mixed, yb.get(), s, err.as<int>());
+            scatter_channels_device(yb.get(), Mb, N, chmap.as<int32_t>() + off[(size_t)k], M, out.ptr, esz, s);
         }
         out.finish(s);
         int herr = 0;

@@ -96,8 +96,8 @@ __device__ __forceinline__ double pow2d(int k) { return __longlong_as_double((lo
 // finite one).  The table must be zero on entry.  Block: 32 channel quads x 8
 // time phases over `seg` rows (seg divides the run length); grid (row
 // segments, channel blocks of 128).
-__global__ void __launch_bounds__(256) cov_run_maxbits(const float* __restrict__ X, int64_t M, int64_t rows,
-                                                       int64_t R, int64_t seg, int64_t Mp,
+__global__ void __launch_bounds__(256) cov_run_maxbits(const float* __restrict__ X, int64_t M, int64_t ld,
+                                                       int64_t rows, int64_t R, int64_t seg, int64_t Mp,
                                                        unsigned int* __restrict__ maxbits) {
     __shared__ unsigned int red[8][kB];
     const int q = threadIdx.x & 31, ph = threadIdx.x >> 5;
@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(256) cov_run_maxbits(const float* __restrict__
         const float* p = X + c0;
 #pragma unroll 8
         for (int64_t t = t0 + ph; t < t1; t += 8) {
-            const float4 v = __ldg(reinterpret_cast<const float4*>(p + t * M));
+            const float4 v = __ldg(reinterpret_cast<const float4*>(p + t * ld));
             mx[0] = max(mx[0], __float_as_uint(v.x) & 0x7FFFFFFFu);
             mx[1] = max(mx[1], __float_as_uint(v.y) & 0x7FFFFFFFu);
             mx[2] = max(mx[2], __float_as_uint(v.z) & 0x7FFFFFFFu);
@@ -594,14 +594,14 @@ size_t cov_i8_partials_bytes(int64_t M, int64_t runs) {
     return (size_t)runs * cov_i8_pairs(M) * kB * kB * sizeof(double);
 }
 
-void cov_i8_partials(const float* X, int64_t M, int64_t r0, int64_t r1, int64_t R, double* partials,
+void cov_i8_partials(const float* X, int64_t M, int64_t ld, int64_t r0, int64_t r1, int64_t R, double* partials,
                      cudaStream_t stream) {
     const int64_t rows = r1 - r0;
     if (rows <= 0 || M <= 0) return;
     if (R <= 0 || R % kKT != 0 || R > 32768)
         throw_invalid("covariance run length must be a multiple of 32, at most 32768");
-    const float* Xr = X + r0 * M;
-    if (M % 4 != 0 || (reinterpret_cast<uintptr_t>(Xr) & 15) != 0)
+    const float* Xr = X + r0 * ld;
+    if (M % 4 != 0 || ld % 4 != 0 || (reinterpret_cast<uintptr_t>(Xr) & 15) != 0)
         throw_invalid("tensor-core covariance needs M % 4 == 0 and 16-byte aligned rows");
     if (rows > 0x7fffffffLL) throw_unsupported("tensor-core covariance: more than 2^31 rows in one call");
     const int nb = (int)ceil_div(M, kB);
@@ -613,11 +613,11 @@ void cov_i8_partials(const float* X, int64_t M, int64_t r0, int64_t r1, int64_t 
     int64_t seg = 1024;  // rows per block of the max pass: a divisor of R
     while (R % seg != 0) seg >>= 1;
     cov_run_maxbits<<<dim3((unsigned)ceil_div(rows, seg), (unsigned)nb), 256, 0, stream>>>(
-        Xr, M, rows, R, seg, Mp, maxbits.as<unsigned int>());
+        Xr, M, ld, rows, R, seg, Mp, maxbits.as<unsigned int>());
     MS3_LAUNCH_CHECK();
     CUtensorMap map;
     const cuuint64_t dims[2] = {(cuuint64_t)M, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)M * sizeof(float)};
+    const cuuint64_t strides[1] = {(cuuint64_t)ld * sizeof(float)};
     const cuuint32_t box[2] = {(cuuint32_t)kB, (cuuint32_t)kKT};
     const cuuint32_t es[2] = {1, 1};
     const CUresult cr = encode_fn_cov()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(Xr), dims,

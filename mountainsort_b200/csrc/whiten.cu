@@ -51,7 +51,8 @@ constexpr int kCT = 64;   // channel tile
 constexpr int kTT = 32;  // timepoints summed in FP32 before the FP64 add (slice granularity)
 constexpr int kTG = 32;   // timepoints per shared-memory stage of cov_partial
 
-__global__ void __launch_bounds__(256) cov_partial(const float* __restrict__ X, int64_t M, int64_t r0, int64_t N,
+__global__ void __launch_bounds__(256) cov_partial(const float* __restrict__ X, int64_t M, int64_t ld, int64_t r0,
+                                                   int64_t N,
                                                    int nb, int64_t tslice, double* __restrict__ partials) {
     __shared__ __align__(16) float As[kTG][kCT];
     __shared__ __align__(16) float Bs[kTG][kCT];
@@ -79,8 +80,8 @@ __global__ void __launch_bounds__(256) cov_partial(const float* __restrict__ X, 
             const int64_t t = t0 + tt;
             const int64_t ma = (int64_t)bi * kCT + c, mb = (int64_t)bj * kCT + c;
             const bool tv = t < t_end;
-            As[tt][c] = (tv && ma < M) ? X[t * M + ma] : 0.f;
-            Bs[tt][c] = (tv && mb < M) ? X[t * M + mb] : 0.f;
+            As[tt][c] = (tv && ma < M) ? X[t * ld + ma] : 0.f;
+            Bs[tt][c] = (tv && mb < M) ? X[t * ld + mb] : 0.f;
         }
         __syncthreads();
 #pragma unroll 8
@@ -119,7 +120,7 @@ __global__ void __launch_bounds__(256) cov_partial(const float* __restrict__ X, 
 // round-to-nearest FMAs per instruction, the same values as two fmaf calls),
 // which halve the issue slots of the inner product.  FP32 runs of kTT
 // timepoints are flushed to FP64, as in cov_partial, so both kernels produce
-// the same FP32 partial sums.  Needs M % 4 == 0 and a 16-byte aligned X.
+// the same FP32 partial sums.  Needs M % 4 == 0, ld % 4 == 0 and a 16-byte aligned X.
 constexpr int kTS = 16;     // timepoints per stage
 constexpr int kStages8 = 3;
 
@@ -143,7 +144,8 @@ __device__ __forceinline__ void fma_f32x2(uint64_t& d, uint64_t a, uint64_t b) {
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
 }
 
-__global__ void __launch_bounds__(64) cov_partial8(const float* __restrict__ X, int64_t M, int64_t r0, int64_t N,
+__global__ void __launch_bounds__(64) cov_partial8(const float* __restrict__ X, int64_t M, int64_t ld, int64_t r0,
+                                                   int64_t N,
                                                    int nb, int64_t tslice, double* __restrict__ partials) {
     __shared__ __align__(16) float As[kStages8][kTS][kCT];
     __shared__ __align__(16) float Bs[kStages8][kTS][kCT];
@@ -169,8 +171,8 @@ __global__ void __launch_bounds__(64) cov_partial8(const float* __restrict__ X, 
             const int64_t t = tb + tt;
             const int64_t ca = (int64_t)bi * kCT + c4, cb = (int64_t)bj * kCT + c4;
             const bool tv = t < t_end;
-            cp_async16(&As[buf][tt][c4], X + (tv && ca < M ? t * M + ca : 0), tv && ca < M);
-            if (!diag) cp_async16(&Bs[buf][tt][c4], X + (tv && cb < M ? t * M + cb : 0), tv && cb < M);
+            cp_async16(&As[buf][tt][c4], X + (tv && ca < M ? t * ld + ca : 0), tv && ca < M);
+            if (!diag) cp_async16(&Bs[buf][tt][c4], X + (tv && cb < M ? t * ld + cb : 0), tv && cb < M);
         }
     };
 
@@ -764,7 +766,7 @@ __device__ __forceinline__ float quantize_1e4(float x) {
 constexpr int kBM = 64, kBN = 64, kBK = 16;
 
 __global__ void __launch_bounds__(256) apply_gemm(const float* __restrict__ X, const float* __restrict__ Wt,
-                                                  int64_t M, int64_t N, double qunit, int round_1e4,
+                                                  int64_t M, int64_t N, int64_t ld, double qunit, int round_1e4,
                                                   void* __restrict__ out) {
     __shared__ __align__(16) float Xs[kBK][kBM + 4];
     __shared__ __align__(16) float Ws[kBK][kBN + 4];
@@ -783,7 +785,7 @@ __global__ void __launch_bounds__(256) apply_gemm(const float* __restrict__ X, c
         for (int e = threadIdx.x; e < kBM * kBK; e += blockDim.x) {
             const int r = e / kBK, kk = e % kBK;
             const int64_t t = t0 + r, k = k0 + kk;
-            Xs[kk][r] = (t < N && k < M) ? X[t * M + k] : 0.f;
+            Xs[kk][r] = (t < N && k < M) ? X[t * ld + k] : 0.f;
             const int64_t n = n0 + r;
             Ws[kk][r] = (n < M && k < M) ? Wt[n * M + k] : 0.f;
         }
@@ -814,9 +816,9 @@ __global__ void __launch_bounds__(256) apply_gemm(const float* __restrict__ X, c
                 // scale_for_quantization (p_whiten.cpp:445-451): (int)(y/q + 0.5)
                 // stored in a float, then written as int16 by the .mda writer.
                 const int32_t iv = x86_double_to_int32(__dadd_rn(__ddiv_rn((double)y, qunit), 0.5));
-                static_cast<int16_t*>(out)[t * M + n] = x86_float_to_int16((float)iv);
+                static_cast<int16_t*>(out)[t * ld + n] = x86_float_to_int16((float)iv);
             } else {
-                static_cast<float*>(out)[t * M + n] = y;
+                static_cast<float*>(out)[t * ld + n] = y;
             }
         }
     }
@@ -824,25 +826,41 @@ __global__ void __launch_bounds__(256) apply_gemm(const float* __restrict__ X, c
 
 // out[t][j] = X[t][ch[j]] for a channel subset (0-based indices, checked by
 // the caller): ms3.compute_whitening_matrix's extract_channels_from_chunk
-// (p_whiten.cpp:421-433) applied to a whole device array.
-__global__ void gather_channels(const float* __restrict__ X, int64_t M, int64_t N, const int32_t* __restrict__ ch,
-                                int64_t M2, float* __restrict__ out) {
-    const int64_t total = N * M2;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t t = i / M2, j = i - t * M2;
-        if (MS3_IN_BOUNDS(ch[j], M, 201)) out[i] = X[t * M + ch[j]];
+// (p_whiten.cpp:421-433) applied to a whole device array.  A block takes groups
+// of rows small enough for 32-bit index arithmetic: a 64-bit division per element
+// bound the flat form (300k rows, 1532 of 1536 channels: 1169 us to gather and 1193
+// to scatter; now 690 and 767).
+constexpr int kGroupElems = 4096;
+__global__ void __launch_bounds__(256) gather_channels(const float* __restrict__ X, int64_t M, int64_t N,
+                                                       const int32_t* __restrict__ ch, int M2, int rows,
+                                                       float* __restrict__ out) {
+    for (int64_t t0 = (int64_t)blockIdx.x * rows; t0 < N; t0 += (int64_t)gridDim.x * rows) {
+        const unsigned n = (unsigned)min((int64_t)rows, N - t0) * (unsigned)M2;
+        const float* Xg = X + t0 * M;
+        float* og = out + t0 * M2;
+#pragma unroll 4
+        for (unsigned e = threadIdx.x; e < n; e += 256) {
+            const unsigned t = e / (unsigned)M2, j = e - t * (unsigned)M2;
+            if (MS3_IN_BOUNDS(ch[j], M, 201)) og[e] = Xg[(int64_t)t * M + ch[j]];
+        }
     }
 }
 
 // out[t][ch[j]] = Y[t][j]: a whitened channel block back into its columns
 // (element size 4 for float32 output, 2 for int16).
 template <class T>
-__global__ void scatter_channels(const T* __restrict__ Y, int64_t M2, int64_t N, const int32_t* __restrict__ ch,
-                                 int64_t M, T* __restrict__ out) {
-    const int64_t total = N * M2;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t t = i / M2, j = i - t * M2;
-        if (MS3_IN_BOUNDS(ch[j], M, 202)) out[t * M + ch[j]] = Y[i];
+__global__ void __launch_bounds__(256) scatter_channels(const T* __restrict__ Y, int M2, int64_t N,
+                                                        const int32_t* __restrict__ ch, int64_t M, int rows,
+                                                        T* __restrict__ out) {
+    for (int64_t t0 = (int64_t)blockIdx.x * rows; t0 < N; t0 += (int64_t)gridDim.x * rows) {
+        const unsigned n = (unsigned)min((int64_t)rows, N - t0) * (unsigned)M2;
+        const T* Yg = Y + t0 * M2;
+        T* og = out + t0 * M;
+#pragma unroll 4
+        for (unsigned e = threadIdx.x; e < n; e += 256) {
+            const unsigned t = e / (unsigned)M2, j = e - t * (unsigned)M2;
+            if (MS3_IN_BOUNDS(ch[j], M, 202)) og[(int64_t)t * M + ch[j]] = Yg[e];
+        }
     }
 }
 
@@ -868,12 +886,13 @@ static int cov_kernel_choice() {
     return v;
 }
 
-CovPlan cov_plan(const float* X, int64_t M) {
+CovPlan cov_plan(const float* X, int64_t M, int64_t ld) {
     CovPlan p;
+    if (ld == 0) ld = M;
     p.M = M;
     p.nb = (int)ceil_div(M, kCT);
     p.npairs = p.nb * (p.nb + 1) / 2;
-    p.vec = (M % 4 == 0) && ((reinterpret_cast<uintptr_t>(X) & 15) == 0);
+    p.vec = (M % 4 == 0) && (ld % 4 == 0) && ((reinterpret_cast<uintptr_t>(X) & 15) == 0);
     const int choice = cov_kernel_choice();
     p.tc = M > 0 && M % 4 == 0 && choice != 1 && (choice == 2 || M >= 128);
     return p;
@@ -898,39 +917,40 @@ size_t cov_partials_bytes(const CovPlan& p, int64_t slices) {
 }
 
 void cov_partials(const float* X, int64_t M, int64_t r0, int64_t r1, const CovPlan& p, double* partials,
-                  int64_t S, cudaStream_t stream) {
+                  int64_t S, cudaStream_t stream, int64_t ld) {
     const int64_t rows = r1 - r0;
     if (rows <= 0 || S <= 0) return;
     if (p.tc) {  // runs of the plan's length: the slicing the streamed forms use too
         const int64_t R = cov_tslice(p, rows);
         if (ceil_div(rows, R) != S) throw_invalid("covariance: slice count does not match the plan");
-        cov_partials_sliced(X, M, r0, r1, p, partials, R, stream);
+        cov_partials_sliced(X, M, r0, r1, p, partials, R, stream, ld);
         return;
     }
-    cov_partials_sliced(X, M, r0, r1, p, partials, ceil_div(ceil_div(rows, S), kTT) * kTT, stream);
+    cov_partials_sliced(X, M, r0, r1, p, partials, ceil_div(ceil_div(rows, S), kTT) * kTT, stream, ld);
 }
 
 void cov_partials_sliced(const float* X, int64_t M, int64_t r0, int64_t r1, const CovPlan& p, double* partials,
-                         int64_t tslice, cudaStream_t stream) {
+                         int64_t tslice, cudaStream_t stream, int64_t ld) {
     const int64_t rows = r1 - r0;
     if (rows <= 0) return;
+    if (ld == 0) ld = M;
     if (tslice <= 0 || tslice % kTT != 0) throw_invalid("covariance slice length must be a multiple of 32");
     if (p.tc) {
-        if ((reinterpret_cast<uintptr_t>(X + r0 * M) & 15) == 0) {
-            cov_i8_partials(X, M, r0, r1, tslice, partials, stream);
+        if (ld % 4 == 0 && (reinterpret_cast<uintptr_t>(X + r0 * ld) & 15) == 0) {
+            cov_i8_partials(X, M, ld, r0, r1, tslice, partials, stream);
         } else {  // the tensor map needs 16-byte aligned rows: work on an aligned copy
             DevBuf copy(sizeof(float) * (size_t)(rows * M), stream);
-            MS3_CUDA(cudaMemcpyAsync(copy.get(), X + r0 * M, sizeof(float) * (size_t)(rows * M),
-                                     cudaMemcpyDeviceToDevice, stream));
-            cov_i8_partials(copy.as<float>(), M, 0, rows, tslice, partials, stream);
+            MS3_CUDA(cudaMemcpy2DAsync(copy.get(), sizeof(float) * (size_t)M, X + r0 * ld, sizeof(float) * (size_t)ld,
+                                       sizeof(float) * (size_t)M, (size_t)rows, cudaMemcpyDeviceToDevice, stream));
+            cov_i8_partials(copy.as<float>(), M, M, 0, rows, tslice, partials, stream);
         }
         return;
     }
     const int64_t S = ceil_div(rows, tslice);
     if (p.vec)
-        cov_partial8<<<dim3(p.npairs, (unsigned)S), 64, 0, stream>>>(X, M, r0, r1, p.nb, tslice, partials);
+        cov_partial8<<<dim3(p.npairs, (unsigned)S), 64, 0, stream>>>(X, M, ld, r0, r1, p.nb, tslice, partials);
     else
-        cov_partial<<<dim3(p.npairs, (unsigned)S), 256, 0, stream>>>(X, M, r0, r1, p.nb, tslice, partials);
+        cov_partial<<<dim3(p.npairs, (unsigned)S), 256, 0, stream>>>(X, M, ld, r0, r1, p.nb, tslice, partials);
     MS3_LAUNCH_CHECK();
 }
 
@@ -958,12 +978,12 @@ void covariance_sum_device(const float* X, int64_t M, int64_t N, double* XXt_sum
     cov_finish(partials.as<double>(), S, p, M, /*N=*/1, XXt_sum, stream);  // N <= 1: no division
 }
 
-void covariance_device(const float* X, int64_t M, int64_t N, double* XXt, cudaStream_t stream) {
+void covariance_device(const float* X, int64_t M, int64_t N, double* XXt, cudaStream_t stream, int64_t ld) {
     if (M <= 0) return;
-    const CovPlan p = cov_plan(X, M);
+    const CovPlan p = cov_plan(X, M, ld);
     const int64_t S = cov_slices(p, N);
     DevBuf partials(cov_partials_bytes(p, S), stream);
-    cov_partials(X, M, 0, N, p, partials.as<double>(), S, stream);
+    cov_partials(X, M, 0, N, p, partials.as<double>(), S, stream, ld);
     cov_finish(partials.as<double>(), S, p, M, N, XXt, stream);
 }
 
@@ -1025,7 +1045,7 @@ void covariance_device_noalloc(const float* X, int64_t M, int64_t N, double* XXt
     S = ceil_div(N, tslice);
     // Every partial tile the reduction reads is written by cov_partial in this
     // call, so nothing left in the array by an earlier call is ever used.
-    cov_partial<<<dim3(npairs, (unsigned)S), 256, 0, stream>>>(X, M, 0, N, nb, tslice, scratch);
+    cov_partial<<<dim3(npairs, (unsigned)S), 256, 0, stream>>>(X, M, M, 0, N, nb, tslice, scratch);
     MS3_LAUNCH_CHECK();
     const int64_t total = (int64_t)npairs * kCT * kCT;
     cov_reduce<<<(unsigned)ceil_div(total, 256), 256, 0, stream>>>(scratch, (int)S, npairs, nb, M, N, XXt);
@@ -1087,12 +1107,12 @@ bool pca_registers(const double* XXt, int64_t M, int count, double* comps, doubl
 }  // namespace
 
 void whitening_matrix_device(const double* XXt, int64_t M, double* W, double* comps, double* sigma,
-                             cudaStream_t stream) {
-    if (M <= 0) return;
+                             cudaStream_t stream, int count) {
+    if (M <= 0 || count <= 0) return;
     if (M > 65535) throw_unsupported("whitening matrix for more than 65535 channels");
     DevBuf cbuf, sbuf;
-    if (!comps) { cbuf.alloc(sizeof(double) * (size_t)(M * M), stream); comps = cbuf.as<double>(); }
-    if (!sigma) { sbuf.alloc(sizeof(double) * (size_t)M, stream); sigma = sbuf.as<double>(); }
+    if (!comps) { cbuf.alloc(sizeof(double) * (size_t)(M * M) * count, stream); comps = cbuf.as<double>(); }
+    if (!sigma) { sbuf.alloc(sizeof(double) * (size_t)M * count, stream); sigma = sbuf.as<double>(); }
 
     // registers hold the working matrix up to 512 channels (MS3GPU_PCA_KERNEL=smem
     // selects the shared-memory kernel, which gives the same values)
@@ -1100,9 +1120,11 @@ void whitening_matrix_device(const double* XXt, int64_t M, double* W, double* co
     const bool force_smem = pk && std::string(pk) == "smem";
     const char* force_global0 = std::getenv("MS3GPU_PCA_ROWS_GLOBAL");
     const bool registers = !force_smem && !(force_global0 && force_global0[0] == '1');
-    if (!registers || !pca_registers(XXt, M, 1, comps, sigma, stream)) pca_launch_smem(XXt, M, comps, sigma, stream);
+    if (!registers || !pca_registers(XXt, M, count, comps, sigma, stream))
+        for (int64_t k = 0; k < count; k++)
+            pca_launch_smem(XXt + k * M * M, M, comps + k * M * M, sigma + k * M, stream);
     const unsigned wt = (unsigned)ceil_div(M, kWT);
-    w_assemble<<<dim3(wt, wt), 256, 0, stream>>>(comps, sigma, (int)M, W);
+    w_assemble<<<dim3(wt, wt, (unsigned)count), 256, 0, stream>>>(comps, sigma, (int)M, W);
     MS3_LAUNCH_CHECK();
 }
 
@@ -1160,35 +1182,47 @@ void pca_launch_smem(const double* XXt, int64_t M, double* comps, double* sigma,
     MS3_LAUNCH_CHECK();
 }
 
+// rows per group and blocks of the two copies above
+static void channel_copy_shape(int64_t M2, int64_t N, int& rows, unsigned& blocks) {
+    if (M2 > 0x7fffffff) throw_unsupported("more than 2^31 channels");
+    rows = (int)std::max<int64_t>(1, kGroupElems / M2);
+    blocks = (unsigned)std::min<int64_t>(ceil_div(N, rows), (int64_t)num_sms() * 32);
+}
+
 void gather_channels_device(const float* X, int64_t M, int64_t N, const int32_t* ch, int64_t M2, float* out,
                             cudaStream_t stream) {
     if (N <= 0 || M2 <= 0) return;
-    const int64_t blocks = std::min<int64_t>(ceil_div(N * M2, 256), (int64_t)num_sms() * 32);
-    gather_channels<<<(unsigned)blocks, 256, 0, stream>>>(X, M, N, ch, M2, out);
+    int rows;
+    unsigned blocks;
+    channel_copy_shape(M2, N, rows, blocks);
+    gather_channels<<<blocks, 256, 0, stream>>>(X, M, N, ch, (int)M2, rows, out);
     MS3_LAUNCH_CHECK();
 }
 
 void scatter_channels_device(const void* Y, int64_t M2, int64_t N, const int32_t* ch, int64_t M, void* out,
                              size_t elem, cudaStream_t stream) {
     if (N <= 0 || M2 <= 0) return;
-    const int64_t blocks = std::min<int64_t>(ceil_div(N * M2, 256), (int64_t)num_sms() * 32);
+    int rows;
+    unsigned blocks;
+    channel_copy_shape(M2, N, rows, blocks);
     if (elem == 2)
-        scatter_channels<int16_t><<<(unsigned)blocks, 256, 0, stream>>>(static_cast<const int16_t*>(Y), M2, N, ch, M,
-                                                                        static_cast<int16_t*>(out));
+        scatter_channels<int16_t><<<blocks, 256, 0, stream>>>(static_cast<const int16_t*>(Y), (int)M2, N, ch, M, rows,
+                                                              static_cast<int16_t*>(out));
     else
-        scatter_channels<float><<<(unsigned)blocks, 256, 0, stream>>>(static_cast<const float*>(Y), M2, N, ch, M,
-                                                                      static_cast<float*>(out));
+        scatter_channels<float><<<blocks, 256, 0, stream>>>(static_cast<const float*>(Y), (int)M2, N, ch, M, rows,
+                                                            static_cast<float*>(out));
     MS3_LAUNCH_CHECK();
 }
 
 void apply_whitening_device(const float* X, int64_t M, int64_t N, const double* W, double quantization_unit,
-                            bool mixed, void* out, cudaStream_t stream, int* err, bool round_1e4) {
+                            bool mixed, void* out, cudaStream_t stream, int* err, bool round_1e4, int64_t ld) {
     if (M <= 0 || N <= 0) return;
+    if (ld == 0) ld = M;
     // MS3GPU_APPLY_FFMA=1 selects the FP32 FMA kernel for the plain form
     const char* ffma = std::getenv("MS3GPU_APPLY_FFMA");
     const bool force_ffma = ffma && ffma[0] == '1';
-    if (apply_tc_supported(X, M, N, out) && (mixed || !force_ffma)) {
-        apply_whitening_tc(X, M, N, W, quantization_unit, /*drain=*/!mixed, out, stream, err, round_1e4);
+    if (apply_tc_supported(X, M, N, out, ld) && (mixed || !force_ffma)) {
+        apply_whitening_tc(X, M, N, W, quantization_unit, /*drain=*/!mixed, out, stream, err, round_1e4, ld);
         return;
     }
     DevBuf wt(sizeof(float) * (size_t)(M * M), stream);
@@ -1196,7 +1230,7 @@ void apply_whitening_device(const float* X, int64_t M, int64_t N, const double* 
     MS3_LAUNCH_CHECK();
     const int64_t blocks = ceil_div(N, kBM) * ceil_div(M, kBN);
     if (blocks > 0x7fffffff) throw_unsupported("too many tiles for the apply kernel");
-    apply_gemm<<<(unsigned)blocks, 256, 0, stream>>>(X, wt.as<float>(), M, N, quantization_unit, round_1e4 ? 1 : 0,
+    apply_gemm<<<(unsigned)blocks, 256, 0, stream>>>(X, wt.as<float>(), M, N, ld, quantization_unit, round_1e4 ? 1 : 0,
                                                      out);
     MS3_LAUNCH_CHECK();
 }

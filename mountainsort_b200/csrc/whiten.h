@@ -7,8 +7,11 @@
 
 namespace ms3gpu {
 
+// Row pitches: `ld` (elements between the rows of X; 0 means M) lets the
+// channels be M adjacent columns of a wider recording.
+
 // XXt (M x M doubles, column-major) = sum_t x_t x_t^T / (N-1 if N > 1).
-void covariance_device(const float* X, int64_t M, int64_t N, double* XXt, cudaStream_t stream);
+void covariance_device(const float* X, int64_t M, int64_t N, double* XXt, cudaStream_t stream, int64_t ld = 0);
 // The same sum over the N rows of X without the division (one shard's part
 // of a recording whose rows are spread over several GPUs).
 void covariance_sum_device(const float* X, int64_t M, int64_t N, double* XXt_sum, cudaStream_t stream);
@@ -25,29 +28,29 @@ struct CovPlan {
     bool tc = false;
     int64_t M = 0;
 };
-CovPlan cov_plan(const float* X, int64_t M);
+CovPlan cov_plan(const float* X, int64_t M, int64_t ld = 0);
 int64_t cov_slices(const CovPlan& p, int64_t rows);
 size_t cov_partials_bytes(const CovPlan& p, int64_t slices);
 void cov_partials(const float* X, int64_t M, int64_t r0, int64_t r1, const CovPlan& p, double* partials,
-                  int64_t S, cudaStream_t stream);
+                  int64_t S, cudaStream_t stream, int64_t ld = 0);
 // The slice length covariance_device uses for `rows` rows (a multiple of 32),
 // and cov_partials with that length given: ceil((r1 - r0) / tslice) slices.
 // A recording streamed in slabs of whole slices, each slab's slices written
 // after the previous slab's, sums to the same XXt bit for bit.
 int64_t cov_tslice(const CovPlan& p, int64_t rows);
 void cov_partials_sliced(const float* X, int64_t M, int64_t r0, int64_t r1, const CovPlan& p, double* partials,
-                         int64_t tslice, cudaStream_t stream);
+                         int64_t tslice, cudaStream_t stream, int64_t ld = 0);
 void cov_finish(const double* partials, int64_t S, const CovPlan& p, int64_t M, int64_t N, double* XXt,
                 cudaStream_t stream);
 
 // Tensor-core covariance pieces (cov_i8.cu): runs of R timepoints (a
 // multiple of 32, at most 32768) of rows [r0, r1) of X, one FP64 partial tile
-// per (run, block pair); finish sums `runs` runs in order.  X + r0 * M must
-// be 16-byte aligned with M % 4 == 0.
+// per (run, block pair); finish sums `runs` runs in order.  X + r0 * ld must
+// be 16-byte aligned with M % 4 == 0 and ld % 4 == 0.
 int cov_i8_pairs(int64_t M);
 int64_t cov_i8_run_length(int64_t M, int64_t rows);
 size_t cov_i8_partials_bytes(int64_t M, int64_t runs);
-void cov_i8_partials(const float* X, int64_t M, int64_t r0, int64_t r1, int64_t R, double* partials,
+void cov_i8_partials(const float* X, int64_t M, int64_t ld, int64_t r0, int64_t r1, int64_t R, double* partials,
                      cudaStream_t stream);
 void cov_i8_finish(const double* partials, int64_t runs, int64_t M, int64_t N, double* XXt, cudaStream_t stream);
 // Raises MS3GPU_ERR_CUDA (after a synchronize) when a tensor-core covariance
@@ -71,9 +74,10 @@ void gather_channels_device(const float* X, int64_t M, int64_t N, const int32_t*
 void scatter_channels_device(const void* Y, int64_t M2, int64_t N, const int32_t* ch, int64_t M, void* out,
                              size_t elem, cudaStream_t stream);
 
-// Power-iteration whitening matrix; comps / sigma may be null.
+// Power-iteration whitening matrix; comps / sigma may be null.  count > 1: as many
+// M x M matrices one after another in XXt, W (and comps, sigma), formed side by side.
 void whitening_matrix_device(const double* XXt, int64_t M, double* W, double* comps, double* sigma,
-                             cudaStream_t stream);
+                             cudaStream_t stream, int count = 1);
 
 // out = quantize(W^T x) per timepoint; out float32, or int16 when
 // quantization_unit > 0.  mixed: tensor-core 3-term TF32 (when the shapes
@@ -81,17 +85,18 @@ void whitening_matrix_device(const double* XXt, int64_t M, double* W, double* co
 // err: optional device flag raised by a timed-out tensor-core pipeline; when
 // null the call checks it itself (synchronising the stream).
 // round_1e4 = false skips the 1e-4 rounding (ms3.whiten_clips, which does
-// not round, p_whiten.cpp:300-345).
+// not round, p_whiten.cpp:300-345).  ld: elements between the rows of X and of
+// out (0 means M).
 void apply_whitening_device(const float* X, int64_t M, int64_t N, const double* W,
                             double quantization_unit, bool mixed, void* out, cudaStream_t stream,
-                            int* err = nullptr, bool round_1e4 = true);
+                            int* err = nullptr, bool round_1e4 = true, int64_t ld = 0);
 
 // Tensor-core (tcgen05, 3-term TF32) apply; apply_tc_supported tells whether
 // the shapes and alignment allow it.
-bool apply_tc_supported(const float* X, int64_t M, int64_t N, const void* out);
+bool apply_tc_supported(const float* X, int64_t M, int64_t N, const void* out, int64_t ld);
 // drain: per-K-block draining of the large products into round-to-nearest
 // FP32 sums (plain form); otherwise one FP32 TMEM accumulator (mixed form).
 void apply_whitening_tc(const float* X, int64_t M, int64_t N, const double* W, double quantization_unit,
-                        bool drain, void* out, cudaStream_t stream, int* err = nullptr, bool round_1e4 = true);
+                        bool drain, void* out, cudaStream_t stream, int* err, bool round_1e4, int64_t ld);
 
 }  // namespace ms3gpu
