@@ -764,8 +764,8 @@ SubFft make_subfft(int n, std::vector<float2>& tw) {
     return P;
 }
 
-size_t smem_bytes_for(int n, int G, int twlen) {
-    return (size_t)2 * n * G * sizeof(float2) + (size_t)twlen * sizeof(float2);
+size_t smem_bytes_for(const SubFft& P, int G) {
+    return ((size_t)2 * P.n * G + (size_t)P.twlen + (size_t)extra_entries(P)) * sizeof(float2);
 }
 
 // Device-resident tables for one (L, filter) combination.
@@ -1014,11 +1014,11 @@ void bandpass_device(const void* raw, int64_t M, int64_t N, void* out, const Ban
     // signals per unit: 16 by default (MS3GPU_BP_LOG2G lowers it, for tuning)
     int log2G = (int)std::min<size_t>(4, env_size("MS3GPU_BP_LOG2G", 4));
     while (log2G > 0 && ((int64_t(1) << (log2G - 1)) >= g.P)) log2G--;
-    while (log2G > 0 && (smem_bytes_for((int)plan->L1, 1 << log2G, plan->P1.twlen) > kSmemBudget ||
-                         smem_bytes_for((int)plan->L2, 1 << log2G, plan->P2.twlen) > kSmemBudget))
+    while (log2G > 0 && (smem_bytes_for(plan->P1, 1 << log2G) > kSmemBudget ||
+                         smem_bytes_for(plan->P2, 1 << log2G) > kSmemBudget))
         log2G--;
-    const size_t sm1 = smem_bytes_for((int)plan->L1, 1 << log2G, plan->P1.twlen);
-    const size_t sm2 = smem_bytes_for((int)plan->L2, 1 << log2G, plan->P2.twlen);
+    const size_t sm1 = smem_bytes_for(plan->P1, 1 << log2G);
+    const size_t sm2 = smem_bytes_for(plan->P2, 1 << log2G);
     if (sm1 > kSmemBudget || sm2 > kSmemBudget)
         throw_unsupported("FFT factors of L=" + std::to_string(L) + " exceed shared memory");
     g.log2G = log2G;
