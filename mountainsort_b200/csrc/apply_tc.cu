@@ -512,7 +512,8 @@ bool apply_tc_supported(const float* X, int64_t M, int64_t N, const void* out, i
 }
 
 void apply_whitening_tc(const float* X, int64_t M, int64_t N, const double* W, double quantization_unit,
-                        bool drain, void* out, cudaStream_t stream, int* ext_err, bool round_1e4, int64_t ld) {
+                        bool drain, void* out, cudaStream_t stream, int* ext_err, bool round_1e4, int64_t ld,
+                        int* host_err) {
     DevBuf wbuf(sizeof(float) * (size_t)(2 * M * M) + 256, stream);
     float* whi = wbuf.as<float>();
     float* wlo = whi + M * M;
@@ -525,6 +526,10 @@ void apply_whitening_tc(const float* X, int64_t M, int64_t N, const double* W, d
     else
         launch_apply_tc<128, false>(X, M, N, ld, whi, wlo, quantization_unit, round_1e4 ? 1 : 0, out, err, stream);
     if (ext_err) return;  // the caller checks the flag once for many calls
+    if (host_err) {  // the caller looks at it after its own synchronisation
+        MS3_CUDA(cudaMemcpyAsync(host_err, err, sizeof(int), cudaMemcpyDeviceToHost, stream));
+        return;
+    }
     int herr = 0;
     MS3_CUDA(cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, stream));
     MS3_CUDA(cudaStreamSynchronize(stream));

@@ -1138,11 +1138,19 @@ void bandpass_device(const void* raw, int64_t M, int64_t N, void* out, const Ban
     }
 }
 
+void bandpass_read_timeout(int* flag, cudaStream_t stream) {
+    MS3_CUDA(cudaMemcpyFromSymbolAsync(flag, g_bp_timeout, sizeof(int), 0, cudaMemcpyDeviceToHost, stream));
+}
+
 void bandpass_check_timeout(cudaStream_t stream) {
     int h = 0;
-    MS3_CUDA(cudaMemcpyFromSymbolAsync(&h, g_bp_timeout, sizeof(int), 0, cudaMemcpyDeviceToHost, stream));
+    bandpass_read_timeout(&h, stream);
     MS3_CUDA(cudaStreamSynchronize(stream));
-    if (h) {
+    bandpass_raise_timeout(h, stream);
+}
+
+void bandpass_raise_timeout(int flag, cudaStream_t stream) {
+    if (flag) {
         const int zero = 0;
         MS3_CUDA(cudaMemcpyToSymbolAsync(g_bp_timeout, &zero, sizeof(int), 0, cudaMemcpyHostToDevice, stream));
         MS3_CUDA(cudaStreamSynchronize(stream));

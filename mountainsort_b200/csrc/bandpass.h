@@ -37,5 +37,8 @@ void bandpass_output_rows(int64_t N, int64_t chunk, int sub, int64_t c_begin, in
 // up; synchronizes `stream`.  Call once the bandpass work is ordered before
 // `stream`.
 void bandpass_check_timeout(cudaStream_t stream);
+// Its two halves: queues a copy of the flag; raises for a flag that was set.
+void bandpass_read_timeout(int* flag, cudaStream_t stream);
+void bandpass_raise_timeout(int flag, cudaStream_t stream);
 
 }  // namespace ms3gpu

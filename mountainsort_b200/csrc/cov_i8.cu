@@ -647,17 +647,25 @@ void cov_i8_finish(const double* partials, int64_t runs, int64_t M, int64_t N, d
     MS3_LAUNCH_CHECK();
 }
 
+void covariance_read_timeout(int* flag, cudaStream_t stream) {
+    MS3_CUDA(cudaMemcpyFromSymbolAsync(flag, g_cov_timeout, sizeof(int), 0, cudaMemcpyDeviceToHost, stream));
+}
+
 void covariance_check_timeout(cudaStream_t stream) {
     int h = 0;
-    MS3_CUDA(cudaMemcpyFromSymbolAsync(&h, g_cov_timeout, sizeof(int), 0, cudaMemcpyDeviceToHost, stream));
+    covariance_read_timeout(&h, stream);
     MS3_CUDA(cudaStreamSynchronize(stream));
-    if (h) {
+    covariance_raise_timeout(h, stream);
+    whitening_check_timeout(stream);
+}
+
+void covariance_raise_timeout(int flag, cudaStream_t stream) {
+    if (flag) {
         const int zero = 0;
         MS3_CUDA(cudaMemcpyToSymbolAsync(g_cov_timeout, &zero, sizeof(int), 0, cudaMemcpyHostToDevice, stream));
         MS3_CUDA(cudaStreamSynchronize(stream));
         throw Error(MS3GPU_ERR_CUDA, "tensor-core covariance: pipeline wait timed out");
     }
-    whitening_check_timeout(stream);
 }
 
 int bounds_site_cov(cudaStream_t s) {

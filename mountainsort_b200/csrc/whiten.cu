@@ -1128,11 +1128,19 @@ void whitening_matrix_device(const double* XXt, int64_t M, double* W, double* co
     MS3_LAUNCH_CHECK();
 }
 
+void whitening_read_timeout(int* flag, cudaStream_t stream) {
+    MS3_CUDA(cudaMemcpyFromSymbolAsync(flag, g_pca_timeout, sizeof(int), 0, cudaMemcpyDeviceToHost, stream));
+}
+
 void whitening_check_timeout(cudaStream_t stream) {
     int h = 0;
-    MS3_CUDA(cudaMemcpyFromSymbolAsync(&h, g_pca_timeout, sizeof(int), 0, cudaMemcpyDeviceToHost, stream));
+    whitening_read_timeout(&h, stream);
     MS3_CUDA(cudaStreamSynchronize(stream));
-    if (h) {
+    whitening_raise_timeout(h, stream);
+}
+
+void whitening_raise_timeout(int flag, cudaStream_t stream) {
+    if (flag) {
         const int zero = 0;
         MS3_CUDA(cudaMemcpyToSymbolAsync(g_pca_timeout, &zero, sizeof(int), 0, cudaMemcpyHostToDevice, stream));
         MS3_CUDA(cudaStreamSynchronize(stream));
@@ -1215,14 +1223,15 @@ void scatter_channels_device(const void* Y, int64_t M2, int64_t N, const int32_t
 }
 
 void apply_whitening_device(const float* X, int64_t M, int64_t N, const double* W, double quantization_unit,
-                            bool mixed, void* out, cudaStream_t stream, int* err, bool round_1e4, int64_t ld) {
+                            bool mixed, void* out, cudaStream_t stream, int* err, bool round_1e4, int64_t ld,
+                            int* host_err) {
     if (M <= 0 || N <= 0) return;
     if (ld == 0) ld = M;
     // MS3GPU_APPLY_FFMA=1 selects the FP32 FMA kernel for the plain form
     const char* ffma = std::getenv("MS3GPU_APPLY_FFMA");
     const bool force_ffma = ffma && ffma[0] == '1';
     if (apply_tc_supported(X, M, N, out, ld) && (mixed || !force_ffma)) {
-        apply_whitening_tc(X, M, N, W, quantization_unit, /*drain=*/!mixed, out, stream, err, round_1e4, ld);
+        apply_whitening_tc(X, M, N, W, quantization_unit, /*drain=*/!mixed, out, stream, err, round_1e4, ld, host_err);
         return;
     }
     DevBuf wt(sizeof(float) * (size_t)(M * M), stream);

@@ -61,6 +61,12 @@ void covariance_check_timeout(cudaStream_t stream);
 // The power-iteration part of covariance_check_timeout.
 void whitening_check_timeout(cudaStream_t stream);
 
+// The halves of the two checks: queue a copy of the flag; raise for one that was set.
+void covariance_read_timeout(int* flag, cudaStream_t stream);
+void covariance_raise_timeout(int flag, cudaStream_t stream);
+void whitening_read_timeout(int* flag, cudaStream_t stream);
+void whitening_raise_timeout(int flag, cudaStream_t stream);
+
 // The same covariance with its partial sums in a fixed 16 MiB device array
 // instead of allocated scratch (X and XXt must be device memory).
 void covariance_device_noalloc(const float* X, int64_t M, int64_t N, double* XXt, cudaStream_t stream);
@@ -83,13 +89,14 @@ void whitening_matrix_device(const double* XXt, int64_t M, double* W, double* co
 // quantization_unit > 0.  mixed: tensor-core 3-term TF32 (when the shapes
 // allow), else FP32 FMA.
 // err: optional device flag raised by a timed-out tensor-core pipeline; when
-// null the call checks it itself (synchronising the stream).
+// null the call keeps one of its own and copies it to host_err on the stream, or,
+// when that is null too, checks it itself (synchronising the stream).
 // round_1e4 = false skips the 1e-4 rounding (ms3.whiten_clips, which does
 // not round, p_whiten.cpp:300-345).  ld: elements between the rows of X and of
 // out (0 means M).
 void apply_whitening_device(const float* X, int64_t M, int64_t N, const double* W,
                             double quantization_unit, bool mixed, void* out, cudaStream_t stream,
-                            int* err = nullptr, bool round_1e4 = true, int64_t ld = 0);
+                            int* err = nullptr, bool round_1e4 = true, int64_t ld = 0, int* host_err = nullptr);
 
 // Tensor-core (tcgen05, 3-term TF32) apply; apply_tc_supported tells whether
 // the shapes and alignment allow it.
@@ -97,6 +104,7 @@ bool apply_tc_supported(const float* X, int64_t M, int64_t N, const void* out, i
 // drain: per-K-block draining of the large products into round-to-nearest
 // FP32 sums (plain form); otherwise one FP32 TMEM accumulator (mixed form).
 void apply_whitening_tc(const float* X, int64_t M, int64_t N, const double* W, double quantization_unit,
-                        bool drain, void* out, cudaStream_t stream, int* err, bool round_1e4, int64_t ld);
+                        bool drain, void* out, cudaStream_t stream, int* err, bool round_1e4, int64_t ld,
+                        int* host_err);
 
 }  // namespace ms3gpu
