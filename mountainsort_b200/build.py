@@ -19,7 +19,7 @@ LIB = os.path.join(HERE, "libms3gpu.so")
 LIB_CHECKED = os.path.join(HERE, "libms3gpu_checked.so")  # -DMS3GPU_BOUNDS_CHECK
 EXE = os.path.join(HERE, "ms3gpu.mp")
 
-CU_SOURCES = ["capi.cu", "bandpass.cu", "whiten.cu", "apply_tc.cu", "pipeline.cu", "stream.cu", "artifacts.cu", "detect.cu", "cov_i8.cu"]
+CU_SOURCES = ["capi.cu", "bandpass.cu", "whiten.cu", "apply_tc.cu", "apply_f16.cu", "pipeline.cu", "stream.cu", "artifacts.cu", "detect.cu", "cov_i8.cu"]
 EXE_SOURCES = ["ms3gpu_main.cpp", "mdaio.cpp"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 

@@ -1,4 +1,8 @@
-// Whitening apply on the 5th-generation tensor cores (tcgen05, TMEM).
+// Whitening apply on the 5th-generation tensor cores (tcgen05, TMEM), kind::tf32: int16
+// output, and float output of more than 2816 channels or at addresses that TMA stores
+// cannot reach.  Other float output is apply_f16.cu's, faster and more exact; int16
+// values are whole numbers that change with the last bit of the sums, so they keep this
+// kernel's.
 //
 // y_t = W^T x_t for every timepoint (p_whiten.cpp:174-183: out[m1] +=
 // in[m2] * W[m1*M + m2]), then the reference's 1e-4 rounding and optional

@@ -260,7 +260,8 @@ int guarded(const char* name, F&& f) {
 void bounds_check_all() {
 #ifdef MS3GPU_BOUNDS_CHECK
     MS3_CUDA(cudaDeviceSynchronize());
-    const int sites[4] = {bounds_site_bandpass(0), bounds_site_whiten(0), bounds_site_apply(0), bounds_site_cov(0)};
+    const int sites[5] = {bounds_site_bandpass(0), bounds_site_whiten(0), bounds_site_apply(0),
+                          bounds_site_apply_f16(0), bounds_site_cov(0)};
     for (int v : sites)
         if (v) throw Error(MS3GPU_ERR_CUDA, "bounds check failed at site " + std::to_string(v));
 #endif

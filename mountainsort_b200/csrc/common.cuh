@@ -75,6 +75,7 @@ static inline int take_bounds_site(cudaStream_t s) {
 int bounds_site_bandpass(cudaStream_t s);
 int bounds_site_whiten(cudaStream_t s);
 int bounds_site_apply(cudaStream_t s);
+int bounds_site_apply_f16(cudaStream_t s);
 int bounds_site_cov(cudaStream_t s);
 
 // Stream-ordered device allocation owned by one call.  Freed on the same

@@ -107,4 +107,10 @@ void apply_whitening_tc(const float* X, int64_t M, int64_t N, const double* W, d
                         bool drain, void* out, cudaStream_t stream, int* err, bool round_1e4, int64_t ld,
                         int* host_err);
 
+// Tensor-core apply with float output from halves of 11 bits (three products,
+// round-to-nearest sums per 64 channels): both precision forms.
+bool apply_f16_supported(const float* X, int64_t M, int64_t N, const void* out, int64_t ld);
+void apply_whitening_f16(const float* X, int64_t M, int64_t N, const double* W, void* out, cudaStream_t stream,
+                         int* err, bool round_1e4, int64_t ld, int* host_err);
+
 }  // namespace ms3gpu
