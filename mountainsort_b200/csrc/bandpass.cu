@@ -69,6 +69,7 @@ struct Geom {
     int64_t N2;          // output timepoints
     int out_i16;
     double qscale;       // 1 / quantization_unit
+    int half_lines;      // int16 input or output: neighbouring groups share 128-byte lines
     int in_i16;          // raw is int16 (converted to float on load, like the reference's reader)
 };
 
@@ -104,15 +105,24 @@ __device__ __forceinline__ float2 load_signal(const void* __restrict__ raw, cons
 
 // Units are ordered group-major: consecutive units are consecutive windows of
 // the same channel group, so the half of a window shared with the previous
-// window is read again while it is still in L2.
+// window is read again while it is still in L2.  For int16 input or output a group's
+// row is half a 128-byte line: two neighbouring groups alternate, so that the second
+// finds its half of each line in L2 (384 int16 channels x 600k: F1 901 us, with whole lines fetched 845).
 struct UnitIdx {
     int64_t c;
     int grp;
 };
 __device__ __forceinline__ UnitIdx unit_index(const Geom& g, int64_t unit) {
     UnitIdx u;
-    u.grp = (int)(unit / g.nwin);
-    u.c = g.c_begin + unit % g.nwin;
+    const int64_t both = g.half_lines ? (int64_t)(g.ngroups / 2) * 2 * g.nwin : 0;  // units of group pairs
+    if (unit < both) {
+        const int64_t r = unit % (2 * g.nwin);
+        u.grp = (int)(unit / (2 * g.nwin)) * 2 + (int)(r & 1);
+        u.c = g.c_begin + (r >> 1);
+    } else {
+        u.grp = (int)(both / g.nwin + (unit - both) / g.nwin);
+        u.c = g.c_begin + (unit - both) % g.nwin;
+    }
     return u;
 }
 
@@ -313,6 +323,24 @@ __device__ __forceinline__ void store_filtered(void* __restrict__ out, const Geo
 //                              writes z[i + q RA]   (natural order)
 // Global loads feed pass 1 directly and pass 2 stores directly.
 
+// A read-only load that brings its whole 128-byte line into L2.
+__device__ __forceinline__ uint32_t load_line(const uint32_t* p) {
+    uint32_t v;
+    asm("ld.global.nc.L2::128B.b32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+
+// Two int16 as floats, the same values as the conversion: with its sign bit flipped, a
+// value's 16 bits under the exponent of 2^23 are the float 2^23 + 32768 + value.  The
+// conversion instructions run at a quarter of the rate of these (byte permutes, adds):
+// 384 int16 channels x 600k, F1 912 us with them, 901 without (float input 670).
+__device__ __forceinline__ float2 floats_of(uint32_t pair) {
+    const uint32_t u = pair ^ 0x80008000u;
+    const float lo = __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7410));
+    const float hi = __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7432));
+    return make_float2(__fadd_rn(lo, -8421376.0f), __fadd_rn(hi, -8421376.0f));
+}
+
 // F1, forward columns of length L1 = RA * RB.
 // LG >= 0 and KL2 > 0 fix log2 G and L2 at compile time (the canonical
 // window with 16 signals per unit), so the index arithmetic folds into
@@ -332,25 +360,43 @@ __global__ void __launch_bounds__(256, 3) bpr_cols_forward(const void* __restric
     const UnitIdx ui = unit_index(g, unit0 + blockIdx.y);
     const int64_t t0 = ui.c * g.chunk - kOverlap + n2;
     const int64_t s0 = (int64_t)ui.grp * G;
-    // interior window of whole channel pairs: plain strided loads, no checks
-    const bool interior = g.paired && g.m_even && s0 + G <= g.P && t0 >= 0 && t0 + (int64_t)(n - 1) * L2 < g.N;
+    // a window inside the recording: strided loads without index checks.  An odd channel
+    // count loads a pair's two channels one by one, and the last group's signals beyond P
+    // are left out by a predicate (63 int16 channels: 340 us a launch of 14 units by the
+    // checked loads, now 214).
+    const bool inside = g.paired && t0 >= 0 && t0 + (int64_t)(n - 1) * L2 < g.N;
     for (int it = threadIdx.x; it < (RB << lg); it += blockDim.x) {
         const int gi = it & (G - 1), i = it >> lg;
         float2 u[RA];
-        if (interior) {
-            const int64_t row0 = (t0 + (int64_t)i * L2) * g.M;
-            const int64_t step = (int64_t)RB * L2 * (g.M / 2);  // pairs per RB window rows
-            if (g.in_i16) {
-                const short2* p = reinterpret_cast<const short2*>(static_cast<const int16_t*>(raw) + row0) + (s0 + gi);
+        if (inside) {
+            const int64_t s = s0 + gi;
+            const int64_t at = (t0 + (int64_t)i * L2) * g.M + 2 * s;  // the pair's first channel
+            const int64_t step = (int64_t)RB * L2 * g.M;              // RB window rows
+            const bool ok = s < g.P;
+            if (g.m_even) {
+                if (g.in_i16) {
+                    const uint32_t* p = reinterpret_cast<const uint32_t*>(static_cast<const int16_t*>(raw) + at);
 #pragma unroll
-                for (int q = 0; q < RA; q++) {
-                    const short2 v = __ldg(p + q * step);
-                    u[q] = make_float2((float)v.x, (float)v.y);
+                    for (int q = 0; q < RA; q++) u[q] = floats_of(ok ? load_line(p + q * (step / 2)) : 0u);
+                } else {
+                    const float2* p = reinterpret_cast<const float2*>(static_cast<const float*>(raw) + at);
+#pragma unroll
+                    for (int q = 0; q < RA; q++) u[q] = ok ? __ldg(p + q * (step / 2)) : make_float2(0.f, 0.f);
                 }
             } else {
-                const float2* p = reinterpret_cast<const float2*>(static_cast<const float*>(raw) + row0) + (s0 + gi);
+                const bool two = 2 * s + 1 < g.M;
+                if (g.in_i16) {
+                    const int16_t* p = static_cast<const int16_t*>(raw) + at;
 #pragma unroll
-                for (int q = 0; q < RA; q++) u[q] = __ldg(p + q * step);
+                    for (int q = 0; q < RA; q++)
+                        u[q] = floats_of((ok ? (uint32_t)(uint16_t)__ldg(p + q * step) : 0u) |
+                                         (two ? (uint32_t)(uint16_t)__ldg(p + q * step + 1) << 16 : 0u));
+                } else {
+                    const float* p = static_cast<const float*>(raw) + at;
+#pragma unroll
+                    for (int q = 0; q < RA; q++)
+                        u[q] = make_float2(ok ? __ldg(p + q * step) : 0.f, two ? __ldg(p + q * step + 1) : 0.f);
+                }
             }
         } else {
 #pragma unroll
@@ -655,13 +701,12 @@ __global__ void __launch_bounds__(256, 3) bpr_cols_inverse(const float2* __restr
     const int64_t s0 = (int64_t)ui.grp * G;
     const int64_t ot_base = (ui.c * g.chunk) / g.sub;
     const int L2 = (int)L2v;
-    // float output of whole channel pairs, no subsampling, the whole chunk
-    // inside the output: the kept window rows n1 in [60000 / L2, (60000 +
-    // chunk) / L2) are exactly q in [kQ0, kQ1) for every item i < RB (checked
-    // on the host for this geometry), so plain strided stores of those q only
+    // no subsampling, the whole chunk inside the output: the kept window rows n1 in
+    // [60000 / L2, (60000 + chunk) / L2] are exactly q in [kQ0, kQ1) for every item i < RB
+    // (checked on the host for this geometry), so plain strided stores of those q only
     constexpr int kQ0 = 4, kQ1 = 12;
-    const bool direct = direct_ok && g.sub == 1 && !g.out_i16 && g.paired && g.m_even && s0 + G <= g.P &&
-                        (ui.c + 1) * g.chunk <= g.N2;
+    const bool direct = direct_ok && g.sub == 1 && g.paired && (ui.c + 1) * g.chunk <= g.N2;
+    const bool pairs_fit = g.m_even && (reinterpret_cast<uintptr_t>(out) & (g.out_i16 ? 3 : 7)) == 0;
     const float2* slab = scratch + (size_t)blockIdx.y * (size_t)(g.L * G);
     for (int it = threadIdx.x; it < (RA << lg); it += blockDim.x) {
         const int gi = it & (G - 1), i = it >> lg;
@@ -693,17 +738,36 @@ __global__ void __launch_bounds__(256, 3) bpr_cols_inverse(const float2* __restr
         }
         RegDft<RA, true>::run(u);
         if (direct) {
-            // kept window rows n1 in [kOverlap / L2, (kOverlap + chunk) / L2) are
-            // exactly q in [q0, q1) for every item i < RB
-            float2* o = reinterpret_cast<float2*>(static_cast<float*>(out) +
-                                                  (ot_base + (int64_t)i * L2 + n2 - kOverlap + (int64_t)kQ0 * RB * L2) *
-                                                      g.M) +
-                        (s0 + gi);
-            const int64_t step = (int64_t)RB * L2 * (g.M / 2);
-            const int64_t e0 = (ot_base + (int64_t)i * L2 + n2 - kOverlap + (int64_t)kQ0 * RB * L2) * (g.M / 2) + s0 + gi;
+            const int64_t s = s0 + gi;
+            const bool two = 2 * s + 1 < g.M;
+            const int64_t step = (int64_t)RB * L2 * g.M;
+            const int64_t at = (ot_base + (int64_t)i * L2 + n2 - kOverlap + (int64_t)kQ0 * RB * L2) * g.M + 2 * s;
+            if (s < g.P) {
 #pragma unroll
-            for (int q = kQ0; q < kQ1; q++)
-                if (MS3_IN_BOUNDS(e0 + (q - kQ0) * step, g.N2 * (g.M / 2), 102)) o[(q - kQ0) * step] = u[q];
+                for (int q = kQ0; q < kQ1; q++) {
+                    const int64_t o = at + (q - kQ0) * step;
+                    if (!MS3_IN_BOUNDS(o + (two ? 1 : 0), g.N2 * g.M, 102)) continue;
+                    if (g.out_i16) {
+                        int16_t* o16 = static_cast<int16_t*>(out) + o;
+                        const int16_t a = x86_float_to_int16((float)((double)u[q].x * g.qscale));
+                        const int16_t b = x86_float_to_int16((float)((double)u[q].y * g.qscale));
+                        if (pairs_fit) {
+                            *reinterpret_cast<short2*>(o16) = make_short2(a, b);
+                        } else {
+                            o16[0] = a;
+                            if (two) o16[1] = b;
+                        }
+                    } else {
+                        float* of = static_cast<float*>(out) + o;
+                        if (pairs_fit) {
+                            *reinterpret_cast<float2*>(of) = u[q];
+                        } else {
+                            of[0] = u[q].x;
+                            if (two) of[1] = u[q].y;
+                        }
+                    }
+                }
+            }
         } else {
 #pragma unroll
             for (int q = 0; q < RA; q++) {
@@ -1009,6 +1073,7 @@ void bandpass_device(const void* raw, int64_t M, int64_t N, void* out, const Ban
     g.sub = sub;
     g.N2 = N2;
     g.out_i16 = out_i16 ? 1 : 0;
+    g.half_lines = in_i16 || out_i16;
     g.qscale = out_i16 ? 1.0 / bp.quantization_unit : 1.0;
     // signals per unit: up to 16, limited by the shared-memory budget
     // signals per unit: 16 by default (MS3GPU_BP_LOG2G lowers it, for tuning)
