@@ -33,13 +33,24 @@
 //   warp 0      TMA: fp32 tiles of 32 timepoints x 128 channels (blocks bi,
 //               bj) into a 3-stage ring
 //   warp 1      TMEM allocation (512 columns: four 128 x 128 int32
-//               accumulators); one thread issues the ten MMAs per stage
+//               accumulators); one thread issues the ten products of a
+//               stage as six MMAs (a diagonal pair's seven as four)
 //   warps 2-17  convert fp32 tiles to the four digit planes in the UMMA
-//               MN-major 128-byte-swizzle layout (3-stage ring)
+//               MN-major 128-byte-swizzle layout (3-stage ring), two groups
+//               of eight taking the stages in turn
 //   warps 18-21 at the end of each run: read the accumulators, combine,
 //               scale, store the run's FP64 partial tile
 // Every mbarrier wait is bounded (tc::mbar_wait); a timeout sets
 // g_cov_timeout, which the host checks after the call.
+//
+// What bounds it: the converters, with the MMAs close behind.  An
+// off-diagonal stage takes 0.85 us, of which its MMAs (105 cycles for a
+// product of 128 x 128 x 32) are 0.55.  With all 16 converter warps on one
+// stage every stage paid its two barrier round trips after one another; in two
+// groups one group's loads and barrier waits lie under the other's arithmetic.
+// MMAs of two planes read plane a once for both.  384 channels x 300 k
+// timepoints: 544 us before, 485 with the groups, 476 with the wide MMAs;
+// 200 x 1.5 M: 1037, 916, 901.
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
@@ -71,7 +82,7 @@ constexpr int kF32Stage = 2 * kF32Bytes;      // blocks bi and bj
 constexpr int kPlaneStage = 2 * 4 * kPlaneBytes;
 constexpr int kConvWarps = 16;
 constexpr int kThreads = (2 + kConvWarps + 4) * 32;  // 704
-static_assert(kKT == 2 * kConvWarps, "each converter thread takes two rows of a stage");
+static_assert(kKT == 2 * kConvWarps, "each thread of a group of half the converter warps takes four rows of a stage");
 static_assert(kS1 == kS2, "the converters walk both rings with one stage counter");
 constexpr int kSentinel = 1000;               // scale exponent of a channel whose run holds inf / NaN
 constexpr size_t kSmemBytes = (size_t)kS1 * kF32Stage + (size_t)kS2 * kPlaneStage + 2 * kB * sizeof(int) +
@@ -151,8 +162,8 @@ __device__ __forceinline__ void digits4(const float4 x, const float (&m8)[4], co
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         const float y1 = __fmaf_rn(xv[i], m8[i], 12582912.0f);  // rint(xs / 256) + 1.5 * 2^23 (one rounding)
-        const float vh = __fsub_rn(y1, 12582912.0f);
-        const float rem = fminf(__fmaf_rn(vh, -256.0f, __fmul_rn(xv[i], m[i])), 127.0f);  // exact, then held
+        const float t = __fmaf_rn(y1, -256.0f, 3221225472.0f);  // -256 rint(xs / 256), exact
+        const float rem = fminf(__fmaf_rn(xv[i], m[i], t), 127.0f);  // exact, then held
         const float y2 = __fadd_rn(rem, 12582912.0f);
         w[i] = __float_as_uint(y1) - 0x3F7F80u;  // + 0x8080 (balanced d1, d2), - 0x400000 (d0 in byte 2)
         lo[i] = __float_as_uint(y2);
@@ -179,8 +190,8 @@ __device__ __forceinline__ int sext8(uint32_t b) { return (int)(int8_t)(uint8_t)
 
 // Shared-memory descriptor of one digit plane: MN-major, 128-byte swizzle,
 // 128 channels (one 128-byte row) x 32 timepoints, 8-row groups 1024 bytes
-// apart (stride byte offset); the leading byte offset (the next 128 channels)
-// is not reached when the MN extent is one swizzle row.
+// apart (stride byte offset); the leading byte offset leads to the next plane,
+// which an operand of 256 columns takes as columns 128 to 255.
 __device__ __forceinline__ uint64_t plane_desc(uint32_t saddr) {
     uint64_t d = 0;
     d |= (uint64_t)((saddr >> 4) & 0x3FFF);
@@ -191,17 +202,21 @@ __device__ __forceinline__ uint64_t plane_desc(uint32_t saddr) {
     return d;
 }
 
-// kind::i8 instruction descriptor: S32 accumulator (2), both operands signed
-// 8-bit (1) and MN-major, M = N = 128.
-constexpr uint32_t kIdescI8 = (2u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
-                              ((uint32_t)(kB >> 3) << 17) | ((uint32_t)(kB >> 4) << 24);
+// kind::i8 instruction descriptors: S32 accumulator (2), both operands signed
+// 8-bit (1) and MN-major, M = 128, N = 128 or two planes of 128.
+constexpr uint32_t idesc_i8(int n) {
+    return (2u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((uint32_t)(n >> 3) << 17) |
+           ((uint32_t)(kB >> 4) << 24);
+}
+constexpr uint32_t kIdescI8 = idesc_i8(kB), kIdescI8x2 = idesc_i8(2 * kB);
 
-__device__ __forceinline__ void mma_i8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
+__device__ __forceinline__ void mma_i8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate,
+                                       uint32_t idesc) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %3, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %4, p;\n\t}\n" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(accumulate), "r"(kIdescI8)
+        "l"(adesc), "l"(bdesc), "r"(accumulate), "r"(idesc)
         : "memory");
 }
 
@@ -213,17 +228,17 @@ template <int NBLK, bool DIAG>
 __device__ __forceinline__ void convert_stage(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, int tg,
                                               int q, const float (&m8)[2][4], const float (&mult)[2][4],
                                               int (&dsum)[4]) {
-    float4 x[NBLK][2];
+    float4 x[NBLK][4];
 #pragma unroll
     for (int b = 0; b < NBLK; b++)
 #pragma unroll
-        for (int h = 0; h < 2; h++)
-            x[b][h] = *reinterpret_cast<const float4*>(src + (size_t)b * kF32Bytes + (tg + 16 * h) * (kB * 4) + q * 16);
+        for (int h = 0; h < 4; h++)
+            x[b][h] = *reinterpret_cast<const float4*>(src + (size_t)b * kF32Bytes + (tg + 8 * h) * (kB * 4) + q * 16);
 #pragma unroll
     for (int b = 0; b < NBLK; b++) {
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int t = tg + 16 * h;
+        for (int h = 0; h < 4; h++) {
+            const int t = tg + 8 * h;
             uint32_t w[4], lo[4];
             digits4(x[b][h], m8[b], mult[b], w, lo);
             const uint32_t p0 = gather_byte<2>(w);
@@ -294,10 +309,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (threadIdx.x == 0) {
         for (int s = 0; s < kS1; s++) {
             tc::mbar_init(&f_full[s], 1);
-            tc::mbar_init(&f_empty[s], kConvWarps);
+            tc::mbar_init(&f_empty[s], kConvWarps / 2);
         }
         for (int s = 0; s < kS2; s++) {
-            tc::mbar_init(&p_full[s], kConvWarps);
+            tc::mbar_init(&p_full[s], kConvWarps / 2);
             tc::mbar_init(&p_empty[s], 1);
         }
         tc::mbar_init(acc_full, 1);
@@ -345,6 +360,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
     } else if (warp == 1) {
         if (lane == 0) {
+            // one thread issues: descriptors of stage 0, advanced by additions
+            const uint64_t d0 = plane_desc(tc::smem_u32(planes));
             int64_t g = 0;
             int gs = 0;        // g % kS2
             uint32_t gph = 0;  // (g / kS2) & 1
@@ -362,28 +379,32 @@ __global__ void __launch_bounds__(kThreads, 1)
                         gph ^= 1u;
                     }
                     tc::tc_fence_after();
-                    const uint32_t pa = tc::smem_u32(planes + (size_t)s * kPlaneStage);
-                    const uint32_t pb = diag ? pa : pa + 4 * kPlaneBytes;
+                    const uint64_t da = d0 + (uint64_t)(s * (kPlaneStage >> 4));
+                    const uint64_t db = diag ? da : da + 4 * (kPlaneBytes >> 4);
                     uint64_t a[4], b[4];
 #pragma unroll
                     for (int k = 0; k < 4; k++) {
-                        a[k] = plane_desc(pa + k * kPlaneBytes);
-                        b[k] = plane_desc(pb + k * kPlaneBytes);
+                        a[k] = da + k * (kPlaneBytes >> 4);
+                        b[k] = db + k * (kPlaneBytes >> 4);
                     }
                     const uint32_t acc0 = (kb != 0);
-                    // a diagonal pair (b = a) skips the transposed halves of
-                    // classes 1 and 3 (d1 d0' = (d0 d1')^T, ...): seven MMAs; the
-                    // drain and the reduction add the transposes back
-                    mma_i8(taddr + 0 * kB, a[0], b[0], acc0);
-                    mma_i8(taddr + 1 * kB, a[0], b[1], acc0);
-                    if (!diag) mma_i8(taddr + 1 * kB, a[1], b[0], 1);
-                    mma_i8(taddr + 2 * kB, a[0], b[2], acc0);
-                    mma_i8(taddr + 2 * kB, a[2], b[0], 1);
-                    mma_i8(taddr + 2 * kB, a[1], b[1], 1);
-                    mma_i8(taddr + 3 * kB, a[0], b[3], acc0);
-                    if (!diag) mma_i8(taddr + 3 * kB, a[3], b[0], 1);
-                    mma_i8(taddr + 3 * kB, a[1], b[2], 1);
-                    if (!diag) mma_i8(taddr + 3 * kB, a[2], b[1], 1);
+                    // Neighbouring planes of b are 256 columns of one operand, and the
+                    // classes of their products with one plane of a are neighbouring
+                    // accumulators: two products per MMA where that holds, A read once.
+                    mma_i8(taddr + 0 * kB, a[0], b[0], acc0, kIdescI8x2);  // classes 0, 1
+                    mma_i8(taddr + 2 * kB, a[0], b[2], acc0, kIdescI8x2);  // 2, 3
+                    if (diag) {
+                        // b = a: the transposed halves of classes 1 and 3 (d1 d0' = (d0
+                        // d1')^T, ...) are left out; the drain and the reduction add the
+                        // transposes back
+                        mma_i8(taddr + 2 * kB, a[1], b[1], 1, kIdescI8x2);  // 2, 3
+                        mma_i8(taddr + 2 * kB, a[2], b[0], 1, kIdescI8);    // 2
+                    } else {
+                        mma_i8(taddr + 1 * kB, a[1], b[0], 1, kIdescI8x2);  // 1, 2
+                        mma_i8(taddr + 3 * kB, a[1], b[2], 1, kIdescI8);    // 3
+                        mma_i8(taddr + 2 * kB, a[2], b[0], 1, kIdescI8x2);  // 2, 3
+                        mma_i8(taddr + 3 * kB, a[3], b[0], 1, kIdescI8);    // 3
+                    }
                     tc::mma_commit(&p_empty[s]);
                 }
                 if (ok) tc::mma_commit(acc_full);
@@ -395,7 +416,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     } else if (warp < 2 + kConvWarps) {
         const int tid = threadIdx.x - 64;
         const int q = tid & 31;   // channel quad within a block: channels 4q .. 4q+3
-        const int tg = tid >> 5;  // rows tg and tg + 16 of each stage
+        // two groups of eight warps take the stages in turn; rows tg + 8 k of the group's
+        const int tg = (tid >> 5) & 7, grp = tid >> 8;
         int64_t g = 0;
         int gs = 0;         // g % kS1 (= g % kS2)
         uint32_t gph = 0;   // (g / kS1) & 1
@@ -419,15 +441,17 @@ __global__ void __launch_bounds__(kThreads, 1)
             int dsum[4] = {0, 0, 0, 0};  // sums of d2^2 per channel (diagonal items)
             for (int kb = 0; kb < it.nkb; kb++, g++) {
                 const int s1 = gs, s2 = gs;
-                ok = tc::mbar_wait(&f_full[s1], gph, err);
-                if (ok && g >= kS2) ok = tc::mbar_wait(&p_empty[s2], gph ^ 1u, err);
-                if (!__all_sync(0xffffffffu, ok)) {
-                    ok = false;
-                    break;
-                }
+                const uint32_t ph = gph;
                 if (++gs == kS1) {  // stage and phase of K-block g + 1
                     gs = 0;
                     gph ^= 1u;
+                }
+                if ((int)(g & 1) != grp) continue;
+                ok = tc::mbar_wait(&f_full[s1], ph, err);
+                if (ok && g >= kS2) ok = tc::mbar_wait(&p_empty[s2], ph ^ 1u, err);
+                if (!__all_sync(0xffffffffu, ok)) {
+                    ok = false;
+                    break;
                 }
                 const uint8_t* src = f32 + (size_t)s1 * kF32Stage;
                 uint8_t* dst = planes + (size_t)s2 * kPlaneStage;
