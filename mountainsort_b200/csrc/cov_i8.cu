@@ -27,14 +27,14 @@
 // ~1e-9), and it does not depend on how the runs are grouped into CTAs or
 // slabs, so a recording streamed in slabs of whole runs gives the same bits.
 //
-// Work items are (run, pair of 128-channel blocks with bi <= bj); a
-// persistent CTA per SM walks items r * P + p so CTAs running at the same
-// time share the run's rows through L2.  Per CTA:
-//   warp 0      TMA: fp32 tiles of 32 timepoints x 128 channels (blocks bi,
-//               bj) into a 3-stage ring
+// Work items are (run, pair of 128-channel blocks with bi <= bj), dealt to one
+// persistent CTA per SM by cov_share.h.  A stage is 32 timepoints of an
+// off-diagonal pair's two blocks or 64 of a diagonal pair's one.  Per CTA:
+//   warp 0      TMA: two fp32 tiles of 32 timepoints x 128 channels a stage
+//               into a 3-stage ring
 //   warp 1      TMEM allocation (512 columns: four 128 x 128 int32
 //               accumulators); one thread issues the ten products of a
-//               stage as six MMAs (a diagonal pair's seven as four)
+//               stage as six MMAs (a diagonal pair's fourteen as eight)
 //   warps 2-17  convert fp32 tiles to the four digit planes in the UMMA
 //               MN-major 128-byte-swizzle layout (3-stage ring), two groups
 //               of eight taking the stages in turn
@@ -43,14 +43,21 @@
 // Every mbarrier wait is bounded (tc::mbar_wait); a timeout sets
 // g_cov_timeout, which the host checks after the call.
 //
-// What bounds it: the converters, with the MMAs close behind.  An
-// off-diagonal stage takes 0.85 us, of which its MMAs (105 cycles for a
-// product of 128 x 128 x 32) are 0.55.  With all 16 converter warps on one
-// stage every stage paid its two barrier round trips after one another; in two
-// groups one group's loads and barrier waits lie under the other's arithmetic.
-// MMAs of two planes read plane a once for both.  384 channels x 300 k
-// timepoints: 544 us before, 485 with the groups, 476 with the wide MMAs;
-// 200 x 1.5 M: 1037, 916, 901.
+// What bounds it: shared memory.  An off-diagonal stage is written there by TMA
+// (32 KB), read and written back as planes by the converters (64 KB) and read
+// by its MMAs (64 KB): 1250 cycles at 128 bytes a cycle, of about 1600 that it
+// takes (0.85 us); a diagonal stage 1440 of about 2300.  Hence MMAs of two planes,
+// which read plane a once for both, and two groups of converter warps, so that
+// one group's barrier round trips lie under the other's arithmetic.  A diagonal
+// stage of 32 timepoints had one tile in flight where there is room for two.
+// One pair for each CTA (a grid that is a multiple of P) left the diagonal
+// pairs' CTAs idle for part of the time, and a last wave with few items.
+//   us                        384 x 300 k   200 x 1.5 M   384 x 1.5 M   128 x 1.2 M
+//   one group, narrow MMAs        544          1037          1883             -
+//   two groups                    485           916          1757           210
+//   wide MMAs                     476           901          1733           198
+//   64-step diagonal stages
+//   and the level deal            387           729          1428           157
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
@@ -62,6 +69,7 @@
 #include <string>
 
 #include "common.cuh"
+#include "cov_share.h"
 #include "ms3gpu.h"
 #include "tc_sm100.cuh"
 #include "whiten.h"
@@ -97,6 +105,9 @@ __host__ __device__ inline void pair_blocks(int p, int nb, int& bi, int& bj) {
     }
     bj = bi + p;
 }
+
+// Pair index of blocks bi <= bj: the inverse of pair_blocks.
+__host__ __device__ inline int pair_index(int bi, int bj, int nb) { return bi * nb - bi * (bi - 1) / 2 + (bj - bi); }
 
 // 2^k as a double (k within the normal range).
 __device__ __forceinline__ double pow2d(int k) { return __longlong_as_double((long long)(1023 + k) << 52); }
@@ -186,8 +197,6 @@ __device__ __forceinline__ void tmem_ld_32x32b_x8(uint32_t taddr, uint32_t (&r)[
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-__device__ __forceinline__ int sext8(uint32_t b) { return (int)(int8_t)(uint8_t)(b & 0xFFu); }
-
 // Shared-memory descriptor of one digit plane: MN-major, 128-byte swizzle,
 // 128 channels (one 128-byte row) x 32 timepoints, 8-row groups 1024 bytes
 // apart (stride byte offset); the leading byte offset leads to the next plane,
@@ -220,10 +229,19 @@ __device__ __forceinline__ void mma_i8(uint32_t tmem_d, uint64_t adesc, uint64_t
         : "memory");
 }
 
-// One stage of the converter warps: thread (tg, q) turns rows tg and tg + 16
-// of each block's fp32 tile (channels 4q .. 4q + 3) into the four digit
-// planes; all its loads are issued before the arithmetic.  DIAG: one block
-// (bi == bj), whose d2^2 sums go to dsum.
+// The seven kept products of one K block of a diagonal pair, planes at `a`.
+__device__ __forceinline__ void diag_products(uint32_t taddr, uint64_t a, uint32_t acc0) {
+    constexpr uint64_t kPl = kPlaneBytes >> 4;
+    mma_i8(taddr + 0 * kB, a, a, acc0, kIdescI8x2);              // classes 0, 1
+    mma_i8(taddr + 2 * kB, a, a + 2 * kPl, acc0, kIdescI8x2);    // 2, 3
+    mma_i8(taddr + 2 * kB, a + kPl, a + kPl, 1, kIdescI8x2);     // 2, 3
+    mma_i8(taddr + 2 * kB, a + 2 * kPl, a, 1, kIdescI8);         // 2
+}
+
+// One stage of the converter warps: thread (tg, q) turns rows tg + 8 h of
+// each fp32 tile (channels 4q .. 4q + 3) into the four digit planes; all its
+// loads are issued before the arithmetic.  DIAG: the tiles are K blocks of one
+// channel block (bi == bj), whose d2^2 sums go to dsum.
 template <int NBLK, bool DIAG>
 __device__ __forceinline__ void convert_stage(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, int tg,
                                               int q, const float (&m8)[2][4], const float (&mult)[2][4],
@@ -236,6 +254,7 @@ __device__ __forceinline__ void convert_stage(const uint8_t* __restrict__ src, u
             x[b][h] = *reinterpret_cast<const float4*>(src + (size_t)b * kF32Bytes + (tg + 8 * h) * (kB * 4) + q * 16);
 #pragma unroll
     for (int b = 0; b < NBLK; b++) {
+        uint32_t d2s[4];
 #pragma unroll
         for (int h = 0; h < 4; h++) {
             const int t = tg + 8 * h;
@@ -245,13 +264,7 @@ __device__ __forceinline__ void convert_stage(const uint8_t* __restrict__ src, u
             const uint32_t p1 = gather_byte<1>(w) ^ 0x80808080u;
             const uint32_t p2 = gather_byte<0>(w) ^ 0x80808080u;
             const uint32_t p3 = gather_byte<0>(lo);
-            if (DIAG) {
-#pragma unroll
-                for (int c = 0; c < 4; c++) {
-                    const int d2 = sext8(p2 >> (8 * c));
-                    dsum[c] += d2 * d2;
-                }
-            }
+            if (DIAG) d2s[h] = p2;
             const int r8 = t & 7;
             const size_t off = (size_t)(t >> 3) * 1024 + r8 * 128 + (((q >> 2) ^ r8) << 4) + ((q & 3) << 2);
             uint8_t* pl = dst + (size_t)b * 4 * kPlaneBytes + off;
@@ -259,6 +272,14 @@ __device__ __forceinline__ void convert_stage(const uint8_t* __restrict__ src, u
             *reinterpret_cast<uint32_t*>(pl + kPlaneBytes) = p1;
             *reinterpret_cast<uint32_t*>(pl + 2 * kPlaneBytes) = p2;
             *reinterpret_cast<uint32_t*>(pl + 3 * kPlaneBytes) = p3;
+        }
+        if (DIAG) {  // d2 of four rows per channel (a 4 x 4 transpose of bytes), squared and summed
+            const uint32_t a01 = __byte_perm(d2s[0], d2s[1], 0x5140), a23 = __byte_perm(d2s[2], d2s[3], 0x5140);
+            const uint32_t b01 = __byte_perm(d2s[0], d2s[1], 0x7362), b23 = __byte_perm(d2s[2], d2s[3], 0x7362);
+            const uint32_t ch[4] = {__byte_perm(a01, a23, 0x5410), __byte_perm(a01, a23, 0x7632),
+                                    __byte_perm(b01, b23, 0x5410), __byte_perm(b01, b23, 0x7632)};
+#pragma unroll
+            for (int c = 0; c < 4; c++) dsum[c] = __dp4a((int)ch[c], (int)ch[c], dsum[c]);
         }
     }
 }
@@ -268,6 +289,9 @@ struct Item {
     int p;       // block pair
     int bi, bj;  // channel blocks
     int nkb;     // K blocks (32 timepoints) in the run
+    bool diag;   // bi == bj: two K blocks to a stage, where an off-diagonal pair's has its two blocks
+    __device__ int stages() const { return diag ? (nkb + 1) / 2 : nkb; }
+    __device__ bool both(int st) const { return !diag || 2 * st + 1 < nkb; }  // both halves of stage st are used
 };
 
 __global__ void __launch_bounds__(kThreads, 1)
@@ -292,17 +316,16 @@ __global__ void __launch_bounds__(kThreads, 1)
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mma_done + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t nitems = nruns * P;
-    const int64_t my_items = (blockIdx.x < nitems) ? (nitems - 1 - blockIdx.x) / gridDim.x + 1 : 0;
+    const CovShare share(nruns, nb, blockIdx.x, gridDim.x);
+    const int64_t my_items = share.items();
     if (my_items == 0) return;
     auto item_of = [&](int64_t i) {
         Item it;
-        const int64_t w = blockIdx.x + i * gridDim.x;
-        it.r = w / P;
-        it.p = (int)(w % P);
-        pair_blocks(it.p, nb, it.bi, it.bj);
+        share.item(i, it.r, it.bi, it.bj);
+        it.p = pair_index(it.bi, it.bj, nb);
         const int64_t len = min(R, rows - it.r * R);
         it.nkb = (int)((len + kKT - 1) / kKT);
+        it.diag = it.bi == it.bj;
         return it;
     };
 
@@ -339,8 +362,8 @@ __global__ void __launch_bounds__(kThreads, 1)
             bool ok = true;
             for (int64_t i = 0; i < my_items && ok; i++) {
                 const Item it = item_of(i);
-                const bool diag = it.bi == it.bj;
-                for (int kb = 0; kb < it.nkb; kb++, g++) {
+                const int nst = it.stages();
+                for (int st = 0; st < nst; st++, g++) {
                     const int s = gs;
                     if (g >= kS1 && !(ok = tc::mbar_wait(&f_empty[s], gph ^ 1u, err))) break;
                     if (++gs == kS1) {
@@ -348,10 +371,11 @@ __global__ void __launch_bounds__(kThreads, 1)
                         gph ^= 1u;
                     }
                     uint8_t* dst = f32 + (size_t)s * kF32Stage;
-                    const int y = (int)(it.r * R + (int64_t)kb * kKT);
-                    tc::mbar_expect_tx(&f_full[s], diag ? kF32Bytes : 2 * kF32Bytes);
+                    const int y = (int)(it.r * R + (int64_t)st * (it.diag ? 2 * kKT : kKT));
+                    const bool both = it.both(st);
+                    tc::mbar_expect_tx(&f_full[s], both ? 2 * kF32Bytes : kF32Bytes);
                     tc::tma_load_2d(dst, &tmX, &f_full[s], it.bi * kB, y);
-                    if (!diag) tc::tma_load_2d(dst + kF32Bytes, &tmX, &f_full[s], it.bj * kB, y);
+                    if (both) tc::tma_load_2d(dst + kF32Bytes, &tmX, &f_full[s], it.bj * kB, it.diag ? y + kKT : y);
                 }
             }
             // no copy may still be landing in shared memory when the CTA exits
@@ -368,10 +392,10 @@ __global__ void __launch_bounds__(kThreads, 1)
             bool ok = true;
             for (int64_t i = 0; i < my_items && ok; i++) {
                 const Item it = item_of(i);
-                const bool diag = it.bi == it.bj;
                 if (i > 0 && !(ok = tc::mbar_wait(acc_free, (uint32_t)((i - 1) & 1), err))) break;
                 tc::tc_fence_after();
-                for (int kb = 0; kb < it.nkb; kb++, g++) {
+                const int nst = it.stages();
+                for (int st = 0; st < nst; st++, g++) {
                     const int s = gs;
                     if (!(ok = tc::mbar_wait(&p_full[s], gph, err))) break;
                     if (++gs == kS2) {
@@ -379,31 +403,26 @@ __global__ void __launch_bounds__(kThreads, 1)
                         gph ^= 1u;
                     }
                     tc::tc_fence_after();
-                    const uint64_t da = d0 + (uint64_t)(s * (kPlaneStage >> 4));
-                    const uint64_t db = diag ? da : da + 4 * (kPlaneBytes >> 4);
-                    uint64_t a[4], b[4];
-#pragma unroll
-                    for (int k = 0; k < 4; k++) {
-                        a[k] = da + k * (kPlaneBytes >> 4);
-                        b[k] = db + k * (kPlaneBytes >> 4);
-                    }
-                    const uint32_t acc0 = (kb != 0);
+                    const uint64_t first = d0 + (uint64_t)(s * (kPlaneStage >> 4));
+                    constexpr uint64_t kPl = kPlaneBytes >> 4;
+                    const uint32_t acc0 = (st != 0);
                     // Neighbouring planes of b are 256 columns of one operand, and the
                     // classes of their products with one plane of a are neighbouring
                     // accumulators: two products per MMA where that holds, A read once.
-                    mma_i8(taddr + 0 * kB, a[0], b[0], acc0, kIdescI8x2);  // classes 0, 1
-                    mma_i8(taddr + 2 * kB, a[0], b[2], acc0, kIdescI8x2);  // 2, 3
-                    if (diag) {
+                    if (it.diag) {
                         // b = a: the transposed halves of classes 1 and 3 (d1 d0' = (d0
                         // d1')^T, ...) are left out; the drain and the reduction add the
                         // transposes back
-                        mma_i8(taddr + 2 * kB, a[1], b[1], 1, kIdescI8x2);  // 2, 3
-                        mma_i8(taddr + 2 * kB, a[2], b[0], 1, kIdescI8);    // 2
+                        diag_products(taddr, first, acc0);
+                        if (it.both(st)) diag_products(taddr, first + 4 * kPl, 1);
                     } else {
-                        mma_i8(taddr + 1 * kB, a[1], b[0], 1, kIdescI8x2);  // 1, 2
-                        mma_i8(taddr + 3 * kB, a[1], b[2], 1, kIdescI8);    // 3
-                        mma_i8(taddr + 2 * kB, a[2], b[0], 1, kIdescI8x2);  // 2, 3
-                        mma_i8(taddr + 3 * kB, a[3], b[0], 1, kIdescI8);    // 3
+                        const uint64_t a = first, b = first + 4 * kPl;
+                        mma_i8(taddr + 0 * kB, a, b, acc0, kIdescI8x2);             // classes 0, 1
+                        mma_i8(taddr + 2 * kB, a, b + 2 * kPl, acc0, kIdescI8x2);   // 2, 3
+                        mma_i8(taddr + 1 * kB, a + kPl, b, 1, kIdescI8x2);          // 1, 2
+                        mma_i8(taddr + 3 * kB, a + kPl, b + 2 * kPl, 1, kIdescI8);  // 3
+                        mma_i8(taddr + 2 * kB, a + 2 * kPl, b, 1, kIdescI8x2);      // 2, 3
+                        mma_i8(taddr + 3 * kB, a + 3 * kPl, b, 1, kIdescI8);        // 3
                     }
                     tc::mma_commit(&p_empty[s]);
                 }
@@ -424,7 +443,6 @@ __global__ void __launch_bounds__(kThreads, 1)
         bool ok = true;
         for (int64_t i = 0; i < my_items && ok; i++) {
             const Item it = item_of(i);
-            const bool diag = it.bi == it.bj;
             float mult[2][4], m8[2][4];
 #pragma unroll
             for (int b = 0; b < 2; b++) {
@@ -439,10 +457,11 @@ __global__ void __launch_bounds__(kThreads, 1)
                 }
             }
             int dsum[4] = {0, 0, 0, 0};  // sums of d2^2 per channel (diagonal items)
-            for (int kb = 0; kb < it.nkb; kb++, g++) {
+            const int nst = it.stages();
+            for (int st = 0; st < nst; st++, g++) {
                 const int s1 = gs, s2 = gs;
                 const uint32_t ph = gph;
-                if (++gs == kS1) {  // stage and phase of K-block g + 1
+                if (++gs == kS1) {  // stage and phase of stage g + 1
                     gs = 0;
                     gph ^= 1u;
                 }
@@ -455,7 +474,9 @@ __global__ void __launch_bounds__(kThreads, 1)
                 }
                 const uint8_t* src = f32 + (size_t)s1 * kF32Stage;
                 uint8_t* dst = planes + (size_t)s2 * kPlaneStage;
-                if (diag)
+                if (it.diag && it.both(st))
+                    convert_stage<2, true>(src, dst, tg, q, m8, mult, dsum);
+                else if (it.diag)
                     convert_stage<1, true>(src, dst, tg, q, m8, mult, dsum);
                 else
                     convert_stage<2, false>(src, dst, tg, q, m8, mult, dsum);
@@ -471,7 +492,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             const int par = (int)(i & 1);
             if (i >= 2) ok = tc::mbar_wait(&corr_free[par], (uint32_t)(((i >> 1) - 1) & 1), err);
             if (!__all_sync(0xffffffffu, ok)) break;
-            if (diag) {
+            if (it.diag) {
 #pragma unroll
                 for (int c = 0; c < 4; c++) atomicAdd(&corr[par * kB + 4 * q + c], dsum[c]);
             }
@@ -651,9 +672,7 @@ void cov_i8_partials(const float* X, int64_t M, int64_t ld, int64_t r0, int64_t 
     MS3_CUDA(cudaFuncSetAttribute(cov_i8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
     const int64_t nitems = nruns * P;
     const int sms = sm_count_cov();
-    // a multiple of P CTAs keeps each CTA on one block pair
-    int64_t grid = (P <= sms) ? (int64_t)(sms / P) * P : sms;
-    grid = std::min<int64_t>(grid, nitems);
+    const int64_t grid = std::min<int64_t>(sms, nitems);
     cov_i8_kernel<<<(unsigned)grid, kThreads, kSmemBytes, stream>>>(map, rows, R, nruns, nb, P, Mp,
                                                                  maxbits.as<unsigned int>(), partials);
     MS3_LAUNCH_CHECK();
