@@ -108,21 +108,28 @@ __device__ __forceinline__ float2 load_signal(const void* __restrict__ raw, cons
 // window is read again while it is still in L2.  For int16 input or output a group's
 // row is half a 128-byte line: two neighbouring groups alternate, so that the second
 // finds its half of each line in L2 (384 int16 channels x 600k: F1 901 us, with whole lines fetched 845).
+// Not for subsampled int16 stores (64 channels, every second timepoint: 2201 us a call
+// as it was, 2227 alternating), and for int16 input alone only where a group's piece of a
+// row is half a line, M a multiple of 32 (700 channels: 3420 and 3475).
 struct UnitIdx {
     int64_t c;
     int grp;
 };
-__device__ __forceinline__ UnitIdx unit_index(const Geom& g, int64_t unit) {
+__device__ __forceinline__ UnitIdx unit_index(const Geom& g, int64_t unit64) {
+    // 32 bits (the divisions are in every block): windows x groups of a call that fits in memory
+    const uint32_t unit = (uint32_t)unit64, nwin = (uint32_t)g.nwin;
     UnitIdx u;
-    const int64_t both = g.half_lines ? (int64_t)(g.ngroups / 2) * 2 * g.nwin : 0;  // units of group pairs
+    const uint32_t both = g.half_lines ? (uint32_t)(g.ngroups / 2) * 2 * nwin : 0;  // units of group pairs
+    uint32_t c;
     if (unit < both) {
-        const int64_t r = unit % (2 * g.nwin);
-        u.grp = (int)(unit / (2 * g.nwin)) * 2 + (int)(r & 1);
-        u.c = g.c_begin + (r >> 1);
+        const uint32_t pair = unit / (2 * nwin), r = unit - pair * 2 * nwin;
+        u.grp = (int)(pair * 2 + (r & 1));
+        c = r >> 1;
     } else {
-        u.grp = (int)(both / g.nwin + (unit - both) / g.nwin);
-        u.c = g.c_begin + (unit - both) % g.nwin;
+        u.grp = (int)(unit / nwin);  // `both` is a multiple of nwin
+        c = unit % nwin;
     }
+    u.c = g.c_begin + c;
     return u;
 }
 
@@ -345,7 +352,12 @@ __device__ __forceinline__ float2 floats_of(uint32_t pair) {
 // LG >= 0 and KL2 > 0 fix log2 G and L2 at compile time (the canonical
 // window with 16 signals per unit), so the index arithmetic folds into
 // constant offsets; LG = -1 reads them from g.
-template <int RA, int RB, int LG, int KL2>
+// FORM says what the host found, so that the other forms are not in the kernel: float
+// pairs, int16 pairs, an odd channel count; 0 takes any.  (One kernel with all of them
+// and a predicate on every load: 64 channels x 3.1 M 2062 us a call, 700 int16 channels
+// kept every third timepoint 3546; before there were other forms 2018 and 3447.)
+enum { kAnyForm = 0, kFloatPairs = 1, kInt16Pairs = 2, kOddCount = 3 };
+template <int RA, int RB, int LG, int KL2, int FORM>
 __global__ void __launch_bounds__(256, 3) bpr_cols_forward(const void* __restrict__ raw, float2* __restrict__ scratch,
                                                         Geom g, const float2* __restrict__ roots, int64_t unit0) {
     constexpr int n = RA * RB;
@@ -364,6 +376,7 @@ __global__ void __launch_bounds__(256, 3) bpr_cols_forward(const void* __restric
     // count loads a pair's two channels one by one, and the last group's signals beyond P
     // are left out by a predicate (63 int16 channels: 340 us a launch of 14 units by the
     // checked loads, now 214).
+    const bool whole = s0 + G <= g.P;
     const bool inside = g.paired && t0 >= 0 && t0 + (int64_t)(n - 1) * L2 < g.N;
     for (int it = threadIdx.x; it < (RB << lg); it += blockDim.x) {
         const int gi = it & (G - 1), i = it >> lg;
@@ -373,15 +386,25 @@ __global__ void __launch_bounds__(256, 3) bpr_cols_forward(const void* __restric
             const int64_t at = (t0 + (int64_t)i * L2) * g.M + 2 * s;  // the pair's first channel
             const int64_t step = (int64_t)RB * L2 * g.M;              // RB window rows
             const bool ok = s < g.P;
-            if (g.m_even) {
-                if (g.in_i16) {
+            if (FORM == kAnyForm ? g.m_even != 0 : FORM != kOddCount) {
+                if (FORM == kAnyForm ? g.in_i16 != 0 : FORM == kInt16Pairs) {
                     const uint32_t* p = reinterpret_cast<const uint32_t*>(static_cast<const int16_t*>(raw) + at);
+                    if (whole) {
 #pragma unroll
-                    for (int q = 0; q < RA; q++) u[q] = floats_of(ok ? load_line(p + q * (step / 2)) : 0u);
+                        for (int q = 0; q < RA; q++) u[q] = floats_of(load_line(p + q * (step / 2)));
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < RA; q++) u[q] = floats_of(ok ? load_line(p + q * (step / 2)) : 0u);
+                    }
                 } else {
                     const float2* p = reinterpret_cast<const float2*>(static_cast<const float*>(raw) + at);
+                    if (whole) {
 #pragma unroll
-                    for (int q = 0; q < RA; q++) u[q] = ok ? __ldg(p + q * (step / 2)) : make_float2(0.f, 0.f);
+                        for (int q = 0; q < RA; q++) u[q] = __ldg(p + q * (step / 2));
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < RA; q++) u[q] = ok ? __ldg(p + q * (step / 2)) : make_float2(0.f, 0.f);
+                    }
                 }
             } else {
                 const bool two = 2 * s + 1 < g.M;
@@ -684,7 +707,10 @@ __global__ void __launch_bounds__(kF2Threads, 1)
 // F3, inverse columns of length L1 = RA * RB (inverse order: radix RB, then
 // radix RA), trim / subsample / quantize, store.
 // LG, KL2 as for bpr_cols_forward.
-template <int RA, int RB, int LG, int KL2>
+// FORM, as the host found: float pairs with direct stores, subsampled (no direct
+// stores), or 0 for any.
+enum { kDirectFloatPairs = 1, kSubsampled = 2 };
+template <int RA, int RB, int LG, int KL2, int FORM>
 __global__ void __launch_bounds__(256, 3) bpr_cols_inverse(const float2* __restrict__ scratch, void* __restrict__ out,
                                                         Geom g, const float2* __restrict__ roots, int64_t unit0,
                                                         int direct_ok) {
@@ -705,8 +731,10 @@ __global__ void __launch_bounds__(256, 3) bpr_cols_inverse(const float2* __restr
     // [60000 / L2, (60000 + chunk) / L2] are exactly q in [kQ0, kQ1) for every item i < RB
     // (checked on the host for this geometry), so plain strided stores of those q only
     constexpr int kQ0 = 4, kQ1 = 12;
-    const bool direct = direct_ok && g.sub == 1 && g.paired && (ui.c + 1) * g.chunk <= g.N2;
-    const bool pairs_fit = g.m_even && (reinterpret_cast<uintptr_t>(out) & (g.out_i16 ? 3 : 7)) == 0;
+    const bool direct = FORM != kSubsampled && direct_ok && g.sub == 1 && g.paired && (ui.c + 1) * g.chunk <= g.N2;
+    const bool whole = s0 + G <= g.P;
+    const bool pairs_fit =
+        FORM == kDirectFloatPairs || (g.m_even && (reinterpret_cast<uintptr_t>(out) & (g.out_i16 ? 3 : 7)) == 0);
     const float2* slab = scratch + (size_t)blockIdx.y * (size_t)(g.L * G);
     for (int it = threadIdx.x; it < (RA << lg); it += blockDim.x) {
         const int gi = it & (G - 1), i = it >> lg;
@@ -739,15 +767,15 @@ __global__ void __launch_bounds__(256, 3) bpr_cols_inverse(const float2* __restr
         RegDft<RA, true>::run(u);
         if (direct) {
             const int64_t s = s0 + gi;
-            const bool two = 2 * s + 1 < g.M;
+            const bool two = FORM == kDirectFloatPairs || 2 * s + 1 < g.M;
             const int64_t step = (int64_t)RB * L2 * g.M;
             const int64_t at = (ot_base + (int64_t)i * L2 + n2 - kOverlap + (int64_t)kQ0 * RB * L2) * g.M + 2 * s;
-            if (s < g.P) {
+            if (whole || s < g.P) {
 #pragma unroll
                 for (int q = kQ0; q < kQ1; q++) {
                     const int64_t o = at + (q - kQ0) * step;
                     if (!MS3_IN_BOUNDS(o + (two ? 1 : 0), g.N2 * g.M, 102)) continue;
-                    if (g.out_i16) {
+                    if (FORM != kDirectFloatPairs && g.out_i16) {
                         int16_t* o16 = static_cast<int16_t*>(out) + o;
                         const int16_t a = x86_float_to_int16((float)((double)u[q].x * g.qscale));
                         const int16_t b = x86_float_to_int16((float)((double)u[q].y * g.qscale));
@@ -1073,7 +1101,7 @@ void bandpass_device(const void* raw, int64_t M, int64_t N, void* out, const Ban
     g.sub = sub;
     g.N2 = N2;
     g.out_i16 = out_i16 ? 1 : 0;
-    g.half_lines = in_i16 || out_i16;
+    g.half_lines = (out_i16 && sub == 1) || (in_i16 && M % 32 == 0);
     g.qscale = out_i16 ? 1.0 / bp.quantization_unit : 1.0;
     // signals per unit: up to 16, limited by the shared-memory budget
     // signals per unit: 16 by default (MS3GPU_BP_LOG2G lowers it, for tuning)
@@ -1110,15 +1138,23 @@ void bandpass_device(const void* raw, int64_t M, int64_t N, void* out, const Ban
             MS3_CUDA(cudaFuncSetAttribute(bp_cols_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
             MS3_CUDA(cudaFuncSetAttribute(bp_rows_filter, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
             MS3_CUDA(cudaFuncSetAttribute(bp_cols_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
-            MS3_CUDA(cudaFuncSetAttribute(bpr_cols_forward<kFastRA, kFastRB, -1, 0>,
+            MS3_CUDA(cudaFuncSetAttribute(bpr_cols_forward<kFastRA, kFastRB, -1, 0, kAnyForm>,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
-            MS3_CUDA(cudaFuncSetAttribute(bpr_cols_forward<kFastRA, kFastRB, 4, kFastL2>,
+            MS3_CUDA(cudaFuncSetAttribute(bpr_cols_forward<kFastRA, kFastRB, 4, kFastL2, kFloatPairs>,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
+            MS3_CUDA(cudaFuncSetAttribute(bpr_cols_forward<kFastRA, kFastRB, 4, kFastL2, kInt16Pairs>,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
+            MS3_CUDA(cudaFuncSetAttribute(bpr_cols_forward<kFastRA, kFastRB, 4, kFastL2, kOddCount>,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
             MS3_CUDA(cudaFuncSetAttribute(bpr_rows_filter<kFastSA, kFastSB>,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
-            MS3_CUDA(cudaFuncSetAttribute(bpr_cols_inverse<kFastRA, kFastRB, -1, 0>,
+            MS3_CUDA(cudaFuncSetAttribute(bpr_cols_inverse<kFastRA, kFastRB, -1, 0, kAnyForm>,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
-            MS3_CUDA(cudaFuncSetAttribute(bpr_cols_inverse<kFastRA, kFastRB, 4, kFastL2>,
+            MS3_CUDA(cudaFuncSetAttribute(bpr_cols_inverse<kFastRA, kFastRB, 4, kFastL2, kAnyForm>,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
+            MS3_CUDA(cudaFuncSetAttribute(bpr_cols_inverse<kFastRA, kFastRB, 4, kFastL2, kDirectFloatPairs>,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
+            MS3_CUDA(cudaFuncSetAttribute(bpr_cols_inverse<kFastRA, kFastRB, 4, kFastL2, kSubsampled>,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
             MS3_CUDA(cudaFuncSetAttribute(bpr_rows_filter_pipe<kFastSA, kFastSB>,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1164,6 +1200,14 @@ void bandpass_device(const void* raw, int64_t M, int64_t N, void* out, const Ban
     // column transform directly when the trim falls on those row boundaries
     const int direct_ok = (plan->fast && kOverlap == 4 * kFastRB * plan->L2 &&
                            chunk == 8 * kFastRB * plan->L2) ? 1 : 0;
+    // the forms of the 16-signal kernels' loads and stores
+    const auto forward4 = !g.m_even ? bpr_cols_forward<kFastRA, kFastRB, 4, kFastL2, kOddCount>
+                          : in_i16  ? bpr_cols_forward<kFastRA, kFastRB, 4, kFastL2, kInt16Pairs>
+                                    : bpr_cols_forward<kFastRA, kFastRB, 4, kFastL2, kFloatPairs>;
+    const bool float_pairs = g.m_even && !out_i16 && (reinterpret_cast<uintptr_t>(out) & 7) == 0;
+    const auto inverse4 = sub > 1 ? bpr_cols_inverse<kFastRA, kFastRB, 4, kFastL2, kSubsampled>
+                          : float_pairs ? bpr_cols_inverse<kFastRA, kFastRB, 4, kFastL2, kDirectFloatPairs>
+                                        : bpr_cols_inverse<kFastRA, kFastRB, 4, kFastL2, kAnyForm>;
     for (int64_t u0 = 0; u0 < units; u0 += per_batch) {
         const int64_t nb = std::min<int64_t>(per_batch, units - u0);
         dim3 g1((unsigned)plan->L2, (unsigned)nb);
@@ -1171,9 +1215,9 @@ void bandpass_device(const void* raw, int64_t M, int64_t N, void* out, const Ban
         float2* sc = scratch.as<float2>();
         if (plan->fast) {
             if (g.log2G == 4)
-                bpr_cols_forward<kFastRA, kFastRB, 4, kFastL2><<<g1, 256, fsm1, stream>>>(raw, sc, g, plan->root1, u0);
+                forward4<<<g1, 256, fsm1, stream>>>(raw, sc, g, plan->root1, u0);
             else
-                bpr_cols_forward<kFastRA, kFastRB, -1, 0><<<g1, 256, fsm1, stream>>>(raw, sc, g, plan->root1, u0);
+                bpr_cols_forward<kFastRA, kFastRB, -1, 0, kAnyForm><<<g1, 256, fsm1, stream>>>(raw, sc, g, plan->root1, u0);
             MS3_LAUNCH_CHECK();
             if (G == F2Pipe<kFastSA, kFastSB>::G && reinterpret_cast<uintptr_t>(sc) % 16 == 0) {
                 const int64_t nrows = nb * plan->L1;
@@ -1186,10 +1230,9 @@ void bandpass_device(const void* raw, int64_t M, int64_t N, void* out, const Ban
             }
             MS3_LAUNCH_CHECK();
             if (g.log2G == 4)
-                bpr_cols_inverse<kFastRA, kFastRB, 4, kFastL2>
-                    <<<g1, 256, fsm1, stream>>>(sc, out, g, plan->root1, u0, direct_ok);
+                inverse4<<<g1, 256, fsm1, stream>>>(sc, out, g, plan->root1, u0, direct_ok);
             else
-                bpr_cols_inverse<kFastRA, kFastRB, -1, 0>
+                bpr_cols_inverse<kFastRA, kFastRB, -1, 0, kAnyForm>
                     <<<g1, 256, fsm1, stream>>>(sc, out, g, plan->root1, u0, direct_ok);
             MS3_LAUNCH_CHECK();
         } else {
