@@ -41,15 +41,24 @@ __global__ void __launch_bounds__(128) artifact_norms(const float* __restrict__ 
         const float* p = X + i * I * M + m;
         double s = 0.0;
         int64_t a = 0;
-        for (; a + kBatch <= I; a += kBatch) {
-            float b[kBatch];
+        float b[kBatch];
+        if (I >= kBatch) {
 #pragma unroll
-            for (int j = 0; j < kBatch; j++) b[j] = __ldg(p + (a + j) * M);
+            for (int j = 0; j < kBatch; j++) b[j] = __ldg(p + j * M);
+        }
+        for (; a + kBatch <= I; a += kBatch) {
+            float c[kBatch];  // the next sixteen, on their way during these additions
+            if (a + 2 * kBatch <= I) {
+#pragma unroll
+                for (int j = 0; j < kBatch; j++) c[j] = __ldg(p + (a + kBatch + j) * M);
+            }
 #pragma unroll
             for (int j = 0; j < kBatch; j++) {
                 const double v = (double)b[j];
                 s = __dadd_rn(s, __dmul_rn(v, v));
             }
+#pragma unroll
+            for (int j = 0; j < kBatch; j++) b[j] = c[j];
         }
         for (; a < I; a++) {
             const double v = (double)p[a * M];
@@ -189,8 +198,9 @@ int64_t mask_out_artifacts_device(const float* X, int64_t M, int64_t N, double t
 
 void artifact_norms_device(const float* X, int64_t M, int64_t I, int64_t nint, double* norms, cudaStream_t stream) {
     if (M <= 0 || nint <= 0) return;
-    const int64_t blocks = std::min<int64_t>(ceil_div(M * nint, 128), (int64_t)sm_count() * 64);
-    artifact_norms<<<(unsigned)blocks, 128, 0, stream>>>(X, M, I, nint, norms);
+    const int threads = M * nint < (int64_t)sm_count() * 128 ? 32 : 128;  // few sums: on more SMs
+    const int64_t blocks = std::min<int64_t>(ceil_div(M * nint, threads), (int64_t)sm_count() * 64);
+    artifact_norms<<<(unsigned)blocks, threads, 0, stream>>>(X, M, I, nint, norms);
     MS3_LAUNCH_CHECK();
 }
 
