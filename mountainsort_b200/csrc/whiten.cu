@@ -13,6 +13,8 @@
 //       so the result agrees with the reference's double sum of float
 //       products to ~1e-10 relative.  Partial tiles are reduced in a fixed
 //       order: repeat runs are bit-identical.
+//   cov_partial_small   the same for up to 32 channels, by 4 x 4 blocks on and above
+//       the diagonal.
 //   pca_reg       the reference's power iteration, FP64, the working matrix in
 //       the registers of one CTA or one cluster of 16 (up to 512 channels)
 //   pca_cluster   the same for more channels, one thread-block

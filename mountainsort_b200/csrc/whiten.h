@@ -86,8 +86,9 @@ void whitening_matrix_device(const double* XXt, int64_t M, double* W, double* co
                              cudaStream_t stream, int count = 1);
 
 // out = quantize(W^T x) per timepoint; out float32, or int16 when
-// quantization_unit > 0.  mixed: tensor-core 3-term TF32 (when the shapes
-// allow), else FP32 FMA.
+// quantization_unit > 0.  Float output on the tensor cores from 11-bit halves where
+// apply_f16_supported; otherwise three TF32 products, drained per K-block or, mixed,
+// accumulated over K, where apply_tc_supported; otherwise FP32 FMA.
 // err: optional device flag raised by a timed-out tensor-core pipeline; when
 // null the call keeps one of its own and copies it to host_err on the stream, or,
 // when that is null too, checks it itself (synchronising the stream).
