@@ -32,7 +32,11 @@ namespace {
 // counts is loads in flight: sixteen per thread, and no thread idle when M is not a
 // multiple of the block (64 channels x 3M, intervals of 2000: 683 us with 128-thread
 // rows and loads as the loop came to them, now 197 us).
+// AHEAD: the next sixteen load during the additions, for few sums (below 512 per SM):
+// 64 channels x 1.6 M 396 us a call without, 312 with; x 3 M, whose sums are enough
+// to hide the loads, 549 and 568.
 constexpr int kBatch = 16;
+template <bool AHEAD>
 __global__ void __launch_bounds__(128) artifact_norms(const float* __restrict__ X, int64_t M, int64_t I, int64_t nint,
                                                       double* __restrict__ norms) {
     const int64_t n = M * nint, step = (int64_t)gridDim.x * blockDim.x;
@@ -42,23 +46,26 @@ __global__ void __launch_bounds__(128) artifact_norms(const float* __restrict__ 
         double s = 0.0;
         int64_t a = 0;
         float b[kBatch];
-        if (I >= kBatch) {
+        if (AHEAD && I >= kBatch) {
 #pragma unroll
             for (int j = 0; j < kBatch; j++) b[j] = __ldg(p + j * M);
         }
         for (; a + kBatch <= I; a += kBatch) {
-            float c[kBatch];  // the next sixteen, on their way during these additions
-            if (a + 2 * kBatch <= I) {
+            float c[kBatch];
+            if (AHEAD ? a + 2 * kBatch <= I : true) {
+                const float* from = p + (AHEAD ? a + kBatch : a) * M;
 #pragma unroll
-                for (int j = 0; j < kBatch; j++) c[j] = __ldg(p + (a + kBatch + j) * M);
+                for (int j = 0; j < kBatch; j++) c[j] = __ldg(from + j * M);
             }
 #pragma unroll
             for (int j = 0; j < kBatch; j++) {
-                const double v = (double)b[j];
+                const double v = (double)(AHEAD ? b[j] : c[j]);
                 s = __dadd_rn(s, __dmul_rn(v, v));
             }
+            if (AHEAD) {
 #pragma unroll
-            for (int j = 0; j < kBatch; j++) b[j] = c[j];
+                for (int j = 0; j < kBatch; j++) b[j] = c[j];
+            }
         }
         for (; a < I; a++) {
             const double v = (double)p[a * M];
@@ -200,7 +207,10 @@ void artifact_norms_device(const float* X, int64_t M, int64_t I, int64_t nint, d
     if (M <= 0 || nint <= 0) return;
     const int threads = M * nint < (int64_t)sm_count() * 128 ? 32 : 128;  // few sums: on more SMs
     const int64_t blocks = std::min<int64_t>(ceil_div(M * nint, threads), (int64_t)sm_count() * 64);
-    artifact_norms<<<(unsigned)blocks, threads, 0, stream>>>(X, M, I, nint, norms);
+    if (M * nint < (int64_t)sm_count() * 512)
+        artifact_norms<true><<<(unsigned)blocks, threads, 0, stream>>>(X, M, I, nint, norms);
+    else
+        artifact_norms<false><<<(unsigned)blocks, threads, 0, stream>>>(X, M, I, nint, norms);
     MS3_LAUNCH_CHECK();
 }
 

@@ -33,3 +33,13 @@ def test_oracles_bits(gpu_lib, ref32, M, N, I, shift):
         _, kept = api.mask_out_artifacts(src, threshold=3.0, interval_size=I, out=dst, return_kept=True)
         np.testing.assert_array_equal(dst.cpu().numpy(), ref)
         assert kept == kept_ref
+
+
+@pytest.mark.parametrize("I", [15, 16, 17, 31, 32, 33, 48])
+@pytest.mark.parametrize("nint", [1183, 1185])  # 64 channels: either side of 512 norm sums per SM
+def test_norm_batches(gpu_lib, ref32, I, nint):
+    X = _data(64, nint * I + 3, I)
+    ref, kept_ref = ref32.mask_out_artifacts(X, threshold=3.0, interval_size=I)
+    out, kept = api.mask_out_artifacts(torch.from_numpy(X).cuda(), threshold=3.0, interval_size=I, return_kept=True)
+    np.testing.assert_array_equal(out.cpu().numpy(), ref)
+    assert kept == kept_ref
