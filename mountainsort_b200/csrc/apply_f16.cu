@@ -92,7 +92,26 @@ constexpr size_t smem_bytes(int BN, int cols) {
     return (size_t)kXStages * (kXBytes + kKBytes) + kWStages * w_stage_bytes(BN) +
            (size_t)n_boxes(BN) * kDrainWarps * kBoxBytes + (size_t)cols * sizeof(float) + kRing * kRows * sizeof(int8_t) + 1024 /*align*/ + 256 /*barriers*/;
 }
-static_assert(smem_bytes(kMaxBN, kMaxCols) <= 232448, "shared memory of one CTA");
+// Channels of a call: equal tiles of up to 192, in steps of 16 (the MMA's N).
+constexpr int kMaxM = kMaxCols - 16 * 16;  // 16 column tiles at most, each padded by less than 16
+__host__ __device__ constexpr int col_tiles(int M) { return (M + kMaxBN - 1) / kMaxBN; }
+__host__ __device__ constexpr int tile_cols(int M) { return ((M + col_tiles(M) - 1) / col_tiles(M) + 15) / 16 * 16; }
+// The most that any accepted M asks for.  Not the largest tile's: up to 176 columns there
+// are two boxes per warp (1024 channels, six tiles of 176: 228,480 bytes; 192 x 16: 228,352).
+constexpr size_t max_smem_bytes() {
+    size_t most = 0;
+    for (int M = 4; M <= kMaxM; M += 4) {
+        const size_t b = smem_bytes(tile_cols(M), col_tiles(M) * tile_cols(M));
+        most = b > most ? b : most;
+    }
+    return most;
+}
+constexpr bool cols_fit() {
+    for (int M = 4; M <= kMaxM; M += 4)
+        if (col_tiles(M) * tile_cols(M) > kMaxCols) return false;
+    return true;
+}
+static_assert(max_smem_bytes() <= 232448 && cols_fit(), "shared memory of one CTA");
 
 // 2^k as a float, k within the normal range
 __device__ __forceinline__ float pow2f(int k) { return __uint_as_float((uint32_t)(127 + k) << 23); }
@@ -558,7 +577,7 @@ void set_kernel_attributes(int dev) {
     auto set = [] {
         for (auto k : {apply_f16_kernel<16>, apply_f16_kernel<32>, apply_f16_kernel<64>, apply_f16_kernel<96>})
             MS3_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)smem_bytes(kMaxBN, kMaxCols)));
+                                          (int)max_smem_bytes()));
         for (const void* k : {(const void*)w_prepare_small, (const void*)w_in_scales, (const void*)w_split_f16})
             MS3_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout,
                                           (int)cudaSharedmemCarveoutMaxShared));
@@ -572,7 +591,7 @@ void set_kernel_attributes(int dev) {
 }  // namespace
 
 bool apply_f16_supported(const float* X, int64_t M, int64_t N, const void* out, int64_t ld) {
-    return apply_tc_supported(X, M, N, out, ld) && M <= kMaxCols - 16 * 16 && (reinterpret_cast<uintptr_t>(out) & 15) == 0 && N < (1LL << 31) - kRows;
+    return apply_tc_supported(X, M, N, out, ld) && M <= kMaxM && (reinterpret_cast<uintptr_t>(out) & 15) == 0 && N < (1LL << 31) - kRows;
 }
 
 void apply_whitening_f16(const float* X, int64_t M, int64_t N, const double* W, void* out, cudaStream_t stream,
@@ -580,9 +599,7 @@ void apply_whitening_f16(const float* X, int64_t M, int64_t N, const double* W, 
     int dev = 0;
     MS3_CUDA(cudaGetDevice(&dev));
     set_kernel_attributes(dev);
-    // equal tiles of up to 192 channels, in steps of 16 (the MMA's N)
-    const int ncb = (int)ceil_div(M, kMaxBN);
-    const int BN = (int)ceil_div(ceil_div(M, ncb), 16) * 16;
+    const int ncb = col_tiles((int)M), BN = tile_cols((int)M);
     const int64_t Kp = ceil_div(M, 8) * 8;  // 16-byte rows
     const int64_t n_in = ceil_div(M, kKB) * kKB;
     const size_t w_elems = (size_t)(M * Kp), n_scales = (size_t)n_in + (size_t)ncb * (size_t)BN;
