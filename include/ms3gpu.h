@@ -72,7 +72,7 @@ typedef struct ms3gpu_bandpass_opts {
 #define MS3GPU_PRECISION_PLAIN 0 /* FP32-faithful apply: parity with the reference (<= 1e-5 rel. L2) */
 #define MS3GPU_PRECISION_MIXED 1 /* <= 1e-4 rel. L2 against the FP64 algorithm: int16 output sums its
                                     three TF32 products over all channels in the tensor core; float
-                                    output is formed as in the plain form where the shapes allow */
+                                    output is formed as in the plain form where the shapes and W allow */
 
 /* Whiten_opts (packages/ms3/p_whiten.h:21-26) plus the arithmetic mode. */
 typedef struct ms3gpu_whiten_opts {

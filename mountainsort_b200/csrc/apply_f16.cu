@@ -11,14 +11,28 @@
 // max_m |W(k, m)| and its row of W divided by it: for a whitening matrix that brings
 // channels of any gain to one size.  Then a timepoint's 64 values of a K-block are
 // scaled so that their largest lies in [2^14, 2^15), a column of W likewise.  x_h = rn(x
-// s), x_l = rn(x s - x_h): 22 bits of every value down to 2^-18 of the largest (2^-40 of
-// the largest below that).  The tensor core's FP32 accumulation rounds toward zero, so
-// each K-block of 64 gets a fresh accumulator -- cross products first, while the sum
-// is small, then the four steps of x_h w_h -- and the drain warps add it, times the
-// row's scale, into round-to-nearest FP32 sums in registers (one FMA: the scale is a
-// power of two).  Unrounded outputs against 64 bits, relative: 1.4e-7 at 384 channels
-// (the TF32 kernel 3.1e-7, its undrained form 2.8e-6), 1.0e-7 at 32 (3.3e-7), the same on
-// channels whose gains differ by 10^6.  So both precision forms take this kernel.
+// s), x_l = rn((x s - x_h) 2^11): 22 bits of every value down to 2^-29 of the largest
+// (2^-51 of the largest below that).  The cross products x_l w_h + x_h w_l form at 2^11
+// times their size, and the first step of x_h w_h scales the accumulator back
+// (scale-input-d).  (Without the 2^11, x_l was subnormal from 2^-18 of the largest on.)
+// The tensor core's FP32 accumulation rounds toward zero, so each K-block of 64 gets a
+// fresh accumulator -- cross products first, while the sum is small, then the four
+// steps of x_h w_h -- and the drain warps add it, times the row's scale, into
+// round-to-nearest FP32 sums in registers (one FMA: the scale is a power of two).
+// Unrounded outputs against 64 bits, relative: 1.4e-7 at 384 channels (the TF32 kernel
+// 3.1e-7, its undrained form 2.8e-6), 1.0e-7 at 32 (3.3e-7), the same on channels whose
+// gains differ by 10^6.  So both precision forms take this kernel.
+//
+// Where a value's bits are cut at 2^-51 of the row's largest, the error goes to every
+// output that the value contributes to, also to one whose weight for that largest value
+// is tiny or zero.  So W decides (split_column): this kernel runs when every weight,
+// after the channels' scales, is at least 2^-30 of its column's largest and of the root
+// of its K-block's sum of squares; then the cut is below 2^-21 of the terms that the output
+// sums, for any x.  Otherwise (an identity, block-diagonal or sparse W) the TF32 kernel
+// runs, which holds each value by itself: both are launched, and the one that W's flag
+// does not name returns at once (300 clips of 32 channels: 3 us of 62).  Whitening matrices of correlated channels have
+// their smallest at 2^-24 (384 channels) to 2^-14 (32); uncorrelated noise, 2^-33 at 200.
+// Only W is looked at, so the same W takes the same kernel in every call and slab.
 // A row that holds an infinity or NaN in a K-block, and a column of W that does, come
 // out NaN, as they do from the TF32 split.
 //
@@ -116,6 +130,18 @@ static_assert(max_smem_bytes() <= 232448 && cols_fit(), "shared memory of one CT
 // 2^k as a float, k within the normal range
 __device__ __forceinline__ float pow2f(int k) { return __uint_as_float((uint32_t)(127 + k) << 23); }
 
+constexpr float kLowScale = 2048.0f;  // 2^11: the low halves' factor
+
+// D = A B + 2^-11 D
+__device__ __forceinline__ void mma_f16_after_cross(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, 1, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p, 11;\n\t}\n" ::"r"(tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(idesc)
+        : "memory");
+}
+
 __device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                         uint32_t accumulate) {
     asm volatile(
@@ -157,7 +183,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     apply_f16_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmWh,
                      const __grid_constant__ CUtensorMap tmWl, const __grid_constant__ CUtensorMap tmOut, int64_t M,
                      int64_t N, int BN, int ncb, int64_t ntiles, const float* __restrict__ in_scale,
-                     const float* __restrict__ col_scale, int round_1e4, int* __restrict__ err) {
+                     const float* __restrict__ col_scale, const int* __restrict__ wide, int round_1e4,
+                     int* __restrict__ err) {
+    if (*wide) return;  // the TF32 kernel's
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const uint32_t w_bytes = (uint32_t)BN * 128u;  // one of W_h, W_l
@@ -263,8 +291,9 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
                 for (int k = 0; k < 4; k++)
                     if (left > 16 * k) mma_f16(acc, xh + 2 * k, wl + 2 * k, idesc, 1);
+                mma_f16_after_cross(acc, xh, wh, idesc);
 #pragma unroll
-                for (int k = 0; k < 4; k++)
+                for (int k = 1; k < 4; k++)
                     if (left > 16 * k) mma_f16(acc, xh + 2 * k, wh + 2 * k, idesc, 1);
                 tc::mma_commit(&done[g & (kRing - 1)]);
                 if (++sx == kXStages) sx = 0, px ^= 1;
@@ -310,7 +339,9 @@ __global__ void __launch_bounds__(kThreads, 1)
                     for (int i = 0; i < 4; i++) {
                         const __half2 hi = __floats2half2_rn(f[2 * i] * s, f[2 * i + 1] * s);
                         const float2 hf = __half22float2(hi);
-                        const __half2 lo = __floats2half2_rn(__fmaf_rn(f[2 * i], s, -hf.x), __fmaf_rn(f[2 * i + 1], s, -hf.y));
+                        // the remainders and their multiples are exact
+                        const __half2 lo = __floats2half2_rn(__fmaf_rn(f[2 * i], s, -hf.x) * kLowScale,
+                                                             __fmaf_rn(f[2 * i + 1], s, -hf.y) * kLowScale);
                         hw[i] = *reinterpret_cast<const uint32_t*>(&hi);
                         lw[i] = *reinterpret_cast<const uint32_t*>(&lo);
                     }
@@ -443,18 +474,27 @@ __device__ __forceinline__ double finite_abs(double w) {  // 0 beyond the float 
     return a < 0x1p128 ? a : 0.0;
 }
 
-// 1 / s for a power of two s
+// 1 / s for a power of two s (2^1023 for 0: those weights are zero)
 __device__ __forceinline__ double inverse_pow2(float s) {
     return __hiloint2double((2046 - (__double2hiint((double)s) >> 20)) << 20, 0);
 }
 
-// Column m1 of W^T divided by the channels' scales, one warp: E = floor(log2 max), the
-// column's scale 2^E, the column times 2^(14 - E) as halves w_h = rn(w), w_l = rn(w -
-// w_h), Kp of them (zeros beyond M).  A column with magnitudes beyond the float range,
-// infinities or NaN gets the scale NaN.
-__device__ __forceinline__ void split_column(const double* __restrict__ w, int64_t M, int64_t Kp,
-                                             const float* in_scale, __half* __restrict__ hi, __half* __restrict__ lo,
-                                             float* __restrict__ col_scale) {
+// Where the halves of W go: FP16 for this kernel, TF32 (as apply_tc.cu forms them) for
+// the other, the scales, and the flag for a W that the other takes.
+struct SplitW {
+    __half *hi, *lo;        // [M][Kp]
+    float *hi32, *lo32;     // [M][M]
+    float *in_scale, *col_scale;
+    int *wide, *err;        // err: null, or cleared
+};
+
+// Column m of W^T divided by the channels' scales, one warp: E = floor(log2 max), the
+// column's scale 2^E, the column times 2^(14 - E) as halves w_h = rn(w), w_l = rn((w -
+// w_h) 2^11), Kp of them (zeros beyond M).  A column with magnitudes beyond the float
+// range, infinities or NaN gets the scale NaN.  *wide is set for a weight below 2^-30 of
+// the column's largest or of its K-block's root sum of squares.
+__device__ __forceinline__ void split_column(const double* __restrict__ w, int64_t m, int64_t M, int64_t Kp,
+                                             const float* in_scale, const SplitW& o) {
     const int l = threadIdx.x & 31;
     double top = 0.0;
     bool finite = true;
@@ -467,21 +507,50 @@ __device__ __forceinline__ void split_column(const double* __restrict__ w, int64
     finite = __all_sync(0xffffffffu, finite);
     const int e = exponent_of(top);
     const double s = __hiloint2double((1023 + 14 - e) << 20, 0);
+    bool small = false;
+    for (int64_t k0 = 0; k0 < M; k0 += kKB) {
+        double a2[2] = {0.0, 0.0};
+        bool counts[2];
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int64_t k = k0 + l + 32 * i;
+            counts[i] = k < M && in_scale[k] != 0.f;
+            if (counts[i]) {
+                const double a = finite_abs(w[k]) * inverse_pow2(in_scale[k]);
+                a2[i] = a * a;
+            }
+        }
+        double sum = a2[0] + a2[1];
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        const double least = 0x1p-60 * fmax(sum, top * top);
+        small |= (counts[0] && a2[0] < least) || (counts[1] && a2[1] < least);
+    }
+    if (small && finite) *o.wide = 1;
+    __half* hi = o.hi + m * Kp;
+    __half* lo = o.lo + m * Kp;
 #pragma unroll 4
     for (int64_t k = l; k < Kp; k += 32) {
         const double x = k < M ? w[k] * inverse_pow2(in_scale[k]) * s : 0.0;
         const __half h = __double2half(x);
         hi[k] = h;
-        lo[k] = __double2half(x - (double)__half2float(h));
+        lo[k] = __double2half((x - (double)__half2float(h)) * (double)kLowScale);
+        if (k < M) {
+            const float h32 = __uint_as_float(tc::cvt_rna_tf32((float)w[k]));
+            o.hi32[m * M + k] = h32;
+            o.lo32[m * M + k] = __uint_as_float(tc::cvt_rna_tf32((float)(w[k] - (double)h32)));
+        }
     }
-    if (l == 0) *col_scale = finite ? pow2f(e) : __uint_as_float(0x7FC00000u);
+    if (l == 0) o.col_scale[m] = finite ? pow2f(e) : __uint_as_float(0x7FC00000u);
 }
 
-// in_scale[k] = 2^floor(log2 max_m |W^T[m][k]|), 1 for a channel without weights and
-// beyond M.  Block: 32 channels x 32 parts of m.
-__global__ void __launch_bounds__(1024) w_in_scales(const double* __restrict__ W, int64_t M, int64_t n_in,
-                                                    float* __restrict__ in_scale) {
+__device__ __forceinline__ float in_scale_of(double top) { return top > 0.0 ? pow2f(exponent_of(top)) : 0.f; }
+
+// in_scale[k] = 2^floor(log2 max_m |W^T[m][k]|), 0 for a channel without weights (so
+// that its values, which no output holds, set no row's scale) and beyond M.  Block: 32
+// channels x 32 parts of m.
+__global__ void __launch_bounds__(1024) w_in_scales(const double* __restrict__ W, int64_t M, int64_t n_in, SplitW o) {
     __shared__ double part[32][33];
+    if (blockIdx.x == 0 && threadIdx.x == 0) *o.wide = 0;
     const int l = threadIdx.x & 31, p = threadIdx.x >> 5;
     const int64_t k = (int64_t)blockIdx.x * 32 + l;
     double top = 0.0;
@@ -493,27 +562,24 @@ __global__ void __launch_bounds__(1024) w_in_scales(const double* __restrict__ W
     __syncthreads();
     // warp p reduces channel p of the block
     top = part[l][p];
-    for (int o = 16; o > 0; o >>= 1) top = fmax(top, __shfl_xor_sync(0xffffffffu, top, o));
+    for (int o16 = 16; o16 > 0; o16 >>= 1) top = fmax(top, __shfl_xor_sync(0xffffffffu, top, o16));
     const int64_t kp = (int64_t)blockIdx.x * 32 + p;
-    if (l == 0 && kp < n_in) in_scale[kp] = pow2f(exponent_of(top));
+    if (l == 0 && kp < n_in) o.in_scale[kp] = in_scale_of(top);
 }
 
-__global__ void __launch_bounds__(128) w_split_f16(const double* __restrict__ W, int64_t M, int64_t Kp,
-                                                   const float* __restrict__ in_scale, __half* __restrict__ hi,
-                                                   __half* __restrict__ lo, float* __restrict__ col_scale,
-                                                   int* __restrict__ clear) {
-    if (clear && blockIdx.x == 0 && threadIdx.x == 0) *clear = 0;
+__global__ void __launch_bounds__(128) w_split_f16(const double* __restrict__ W, int64_t M, int64_t Kp, SplitW o) {
+    if (o.err && blockIdx.x == 0 && threadIdx.x == 0) *o.err = 0;
     const int64_t m = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
-    if (m < M) split_column(W + m * M, M, Kp, in_scale, hi + m * Kp, lo + m * Kp, col_scale + m);
+    if (m < M) split_column(W + m * M, m, M, Kp, o.in_scale, o);
 }
 
 // Both in one block for up to 64 channels, where a launch costs more than the work.
 constexpr int kSmallM = 64;
-__global__ void __launch_bounds__(1024) w_prepare_small(const double* __restrict__ W, int M, int Kp,
-                                                        float* __restrict__ in_scale, __half* __restrict__ hi,
-                                                        __half* __restrict__ lo, float* __restrict__ col_scale,
-                                                        int* __restrict__ clear) {
-    if (clear && threadIdx.x == 0) *clear = 0;
+__global__ void __launch_bounds__(1024) w_prepare_small(const double* __restrict__ W, int M, int Kp, SplitW o) {
+    if (threadIdx.x == 0) {
+        *o.wide = 0;
+        if (o.err) *o.err = 0;
+    }
     __shared__ double part[16][kSmallM];
     __shared__ double copy[kSmallM * kSmallM];
     __shared__ float scale[kSmallM];
@@ -534,11 +600,10 @@ __global__ void __launch_bounds__(1024) w_prepare_small(const double* __restrict
     __syncthreads();
     if (p == 0) {
         for (int i = 1; i < 16; i++) top = fmax(top, part[i][k]);
-        in_scale[k] = scale[k] = pow2f(exponent_of(top));
+        o.in_scale[k] = scale[k] = in_scale_of(top);
     }
     __syncthreads();
-    for (int m = threadIdx.x >> 5; m < M; m += 32)
-        split_column(copy + m * M, M, Kp, scale, hi + m * Kp, lo + m * Kp, col_scale + m);
+    for (int m = threadIdx.x >> 5; m < M; m += 32) split_column(copy + m * M, m, M, Kp, scale, o);
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn_f16() {
@@ -594,37 +659,42 @@ bool apply_f16_supported(const float* X, int64_t M, int64_t N, const void* out, 
     return apply_tc_supported(X, M, N, out, ld) && M <= kMaxM && (reinterpret_cast<uintptr_t>(out) & 15) == 0 && N < (1LL << 31) - kRows;
 }
 
-void apply_whitening_f16(const float* X, int64_t M, int64_t N, const double* W, void* out, cudaStream_t stream,
-                         int* ext_err, bool round_1e4, int64_t ld, int* host_err) {
+void apply_whitening_f16(const float* X, int64_t M, int64_t N, const double* W, bool drain, void* out,
+                         cudaStream_t stream, int* ext_err, bool round_1e4, int64_t ld, int* host_err) {
     int dev = 0;
     MS3_CUDA(cudaGetDevice(&dev));
     set_kernel_attributes(dev);
     const int ncb = col_tiles((int)M), BN = tile_cols((int)M);
     const int64_t Kp = ceil_div(M, 8) * 8;  // 16-byte rows
     const int64_t n_in = ceil_div(M, kKB) * kKB;
-    const size_t w_elems = (size_t)(M * Kp), n_scales = (size_t)n_in + (size_t)ncb * (size_t)BN;
-    const size_t w_bytes = (w_elems * sizeof(__half) + 255) / 256 * 256;
-    DevBuf buf(2 * w_bytes + n_scales * sizeof(float) + 256, stream);
-    __half* hi = buf.as<__half>();
-    __half* lo = reinterpret_cast<__half*>(buf.as<char>() + w_bytes);
-    float* scales = reinterpret_cast<float*>(buf.as<char>() + 2 * w_bytes);
-    int* err = ext_err ? ext_err : reinterpret_cast<int*>(scales + n_scales);
-    int* clear = ext_err ? nullptr : err;  // the call's own flag: cleared with the preparation of W
-    float* in_scale = scales;
-    float* col_scale = scales + n_in;
+    const size_t n_scales = (size_t)n_in + (size_t)ncb * (size_t)BN;
+    auto padded = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
+    const size_t half_bytes = padded((size_t)(M * Kp) * sizeof(__half)), tf32_bytes = padded((size_t)(M * M) * sizeof(float));
+    DevBuf buf(2 * half_bytes + 2 * tf32_bytes + n_scales * sizeof(float) + 256, stream);
+    SplitW w;
+    char* at = buf.as<char>();
+    w.hi = reinterpret_cast<__half*>(at);
+    w.lo = reinterpret_cast<__half*>(at += half_bytes);
+    w.hi32 = reinterpret_cast<float*>(at += half_bytes);
+    w.lo32 = reinterpret_cast<float*>(at += tf32_bytes);
+    w.in_scale = reinterpret_cast<float*>(at += tf32_bytes);
+    w.col_scale = w.in_scale + n_in;
+    w.wide = reinterpret_cast<int*>(w.in_scale + n_scales);
+    w.err = ext_err ? nullptr : w.wide + 1;  // the call's own flag: cleared with the preparation of W
+    int* err = ext_err ? ext_err : w.err;
     if (M <= kSmallM) {
-        w_prepare_small<<<1, 1024, 0, stream>>>(W, (int)M, (int)Kp, in_scale, hi, lo, col_scale, clear);
+        w_prepare_small<<<1, 1024, 0, stream>>>(W, (int)M, (int)Kp, w);
     } else {
-        w_in_scales<<<(unsigned)ceil_div(n_in, 32), 1024, 0, stream>>>(W, M, n_in, in_scale);
+        w_in_scales<<<(unsigned)ceil_div(n_in, 32), 1024, 0, stream>>>(W, M, n_in, w);
         MS3_LAUNCH_CHECK();
-        w_split_f16<<<(unsigned)ceil_div(M, 4), 128, 0, stream>>>(W, M, Kp, in_scale, hi, lo, col_scale, clear);
+        w_split_f16<<<(unsigned)ceil_div(M, 4), 128, 0, stream>>>(W, M, Kp, w);
     }
     MS3_LAUNCH_CHECK();
     const CUtensorMap mx = matrix_map(CU_TENSOR_MAP_DATA_TYPE_FLOAT32, X, (uint64_t)M, (uint64_t)N,
                                       (uint64_t)ld * sizeof(float), 32, kRows, CU_TENSOR_MAP_SWIZZLE_128B);
-    const CUtensorMap mh = matrix_map(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, hi, (uint64_t)Kp, (uint64_t)M,
+    const CUtensorMap mh = matrix_map(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, w.hi, (uint64_t)Kp, (uint64_t)M,
                                       (uint64_t)Kp * sizeof(__half), kKB, (uint32_t)BN, CU_TENSOR_MAP_SWIZZLE_128B);
-    const CUtensorMap ml = matrix_map(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, lo, (uint64_t)Kp, (uint64_t)M,
+    const CUtensorMap ml = matrix_map(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, w.lo, (uint64_t)Kp, (uint64_t)M,
                                       (uint64_t)Kp * sizeof(__half), kKB, (uint32_t)BN, CU_TENSOR_MAP_SWIZZLE_128B);
     const CUtensorMap mo = matrix_map(CU_TENSOR_MAP_DATA_TYPE_FLOAT32, out, (uint64_t)M, (uint64_t)N,
                                       (uint64_t)ld * sizeof(float), kBoxCols, 32, CU_TENSOR_MAP_SWIZZLE_64B);
@@ -637,9 +707,10 @@ void apply_whitening_f16(const float* X, int64_t M, int64_t N, const double* W, 
                 : cols <= 32 ? apply_f16_kernel<32>
                 : cols <= 64 ? apply_f16_kernel<64>
                              : apply_f16_kernel<96>;
-    kern<<<(unsigned)std::min<int64_t>(ntiles, nsm), kThreads, sm, stream>>>(mx, mh, ml, mo, M, N, BN, ncb, ntiles, in_scale,
-                                                                            col_scale, round_1e4 ? 1 : 0, err);
+    kern<<<(unsigned)std::min<int64_t>(ntiles, nsm), kThreads, sm, stream>>>(
+        mx, mh, ml, mo, M, N, BN, ncb, ntiles, w.in_scale, w.col_scale, w.wide, round_1e4 ? 1 : 0, err);
     MS3_LAUNCH_CHECK();
+    apply_tc_launch(X, M, N, ld, w.hi32, w.lo32, /*quantization_unit=*/0.0, drain, round_1e4, out, err, w.wide, stream);
     if (ext_err) return;  // the caller checks the flag once for many calls
     if (host_err) {  // the caller looks at it after its own synchronisation
         MS3_CUDA(cudaMemcpyAsync(host_err, err, sizeof(int), cudaMemcpyDeviceToHost, stream));

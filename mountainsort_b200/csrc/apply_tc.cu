@@ -1,8 +1,8 @@
 // Whitening apply on the 5th-generation tensor cores (tcgen05, TMEM), kind::tf32: int16
-// output, and float output of more than 2816 channels or at addresses that TMA stores
-// cannot reach.  Other float output is apply_f16.cu's, faster and more exact; int16
-// values are whole numbers that change with the last bit of the sums, so they keep this
-// kernel's.
+// output, and float output of more than 2816 channels, at addresses that TMA stores
+// cannot reach, or by a matrix whose weights span too wide a range for apply_f16.cu.
+// Other float output is that kernel's, faster and more exact; int16 values are whole
+// numbers that change with the last bit of the sums, so they keep this kernel's.
 //
 // y_t = W^T x_t for every timepoint (p_whiten.cpp:174-183: out[m1] +=
 // in[m2] * W[m1*M + m2]), then the reference's 1e-4 rounding and optional
@@ -187,7 +187,8 @@ __global__ void __launch_bounds__(TcCfg<BN, DRAIN>::kThreads, 1)
     apply_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmWhi,
                     const __grid_constant__ CUtensorMap tmWlo, const __grid_constant__ CUtensorMap tmOut, int out_tma,
                     int64_t M, int64_t N, int64_t ld, int ncb, int64_t ntiles, double qunit, int round_1e4,
-                    void* __restrict__ out, int* __restrict__ err) {
+                    void* __restrict__ out, const int* __restrict__ only_if, int* __restrict__ err) {
+    if (only_if && !*only_if) return;
     using C = TcCfg<BN, DRAIN>;
     constexpr int S = C::kStages;
     constexpr int R = 2;  // accumulator ring (K-blocks when DRAIN, tiles when mixed)
@@ -481,12 +482,28 @@ CUtensorMap make_map(const void* base, uint64_t cols, uint64_t rows, uint64_t ld
     return m;
 }
 
+// Per device, once.
+void set_kernel_attributes(int dev) {
+    static std::once_flag once[64];
+    auto set = [] {
+        MS3_CUDA(cudaFuncSetAttribute(apply_tc_kernel<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)TcCfg<128, true>::kSmemBytes));
+        MS3_CUDA(cudaFuncSetAttribute(apply_tc_kernel<128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)TcCfg<128, false>::kSmemBytes));
+    };
+    if (dev < 64)
+        std::call_once(once[dev], set);
+    else
+        set();
+}
+
 template <int BN, bool DRAIN>
 void launch_apply_tc(const float* X, int64_t M, int64_t N, int64_t ld, const float* whi, const float* wlo, double qunit,
-                     int round_1e4, void* out, int* err, cudaStream_t stream) {
+                     int round_1e4, void* out, int* err, const int* only_if, cudaStream_t stream) {
     using C = TcCfg<BN, DRAIN>;
-    MS3_CUDA(cudaFuncSetAttribute(apply_tc_kernel<BN, DRAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)C::kSmemBytes));
+    int dev = 0, nsm = 0;
+    MS3_CUDA(cudaGetDevice(&dev));
+    set_kernel_attributes(dev);
     const CUtensorMap mx = make_map(X, (uint64_t)M, (uint64_t)N, (uint64_t)ld, kTM);
     const CUtensorMap mh = make_map(whi, (uint64_t)M, (uint64_t)M, (uint64_t)M, BN);
     const CUtensorMap ml = make_map(wlo, (uint64_t)M, (uint64_t)M, (uint64_t)M, BN);
@@ -495,17 +512,24 @@ void launch_apply_tc(const float* X, int64_t M, int64_t N, int64_t ld, const flo
     const CUtensorMap mo = out_tma ? make_map(out, (uint64_t)M, (uint64_t)N, (uint64_t)ld, 32) : mx;
     const int ncb = (int)ceil_div(M, BN);
     const int64_t ntiles = ceil_div(N, kTM) * ncb;
-    int dev = 0, nsm = 0;
-    MS3_CUDA(cudaGetDevice(&dev));
     MS3_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     const int64_t grid = std::min<int64_t>(ntiles, nsm);  // one persistent CTA per SM
     apply_tc_kernel<BN, DRAIN><<<(unsigned)grid, C::kThreads, C::kSmemBytes, stream>>>(mx, mh, ml, mo, out_tma, M, N, ld, ncb,
                                                                                      ntiles, qunit, round_1e4,
-                                                                                     out, err);
+                                                                                     out, only_if, err);
     MS3_LAUNCH_CHECK();
 }
 
 }  // namespace
+
+void apply_tc_launch(const float* X, int64_t M, int64_t N, int64_t ld, const float* whi, const float* wlo,
+                     double quantization_unit, bool drain, bool round_1e4, void* out, int* err, const int* only_if,
+                     cudaStream_t stream) {
+    if (drain)
+        launch_apply_tc<128, true>(X, M, N, ld, whi, wlo, quantization_unit, round_1e4 ? 1 : 0, out, err, only_if, stream);
+    else
+        launch_apply_tc<128, false>(X, M, N, ld, whi, wlo, quantization_unit, round_1e4 ? 1 : 0, out, err, only_if, stream);
+}
 
 bool apply_tc_supported(const float* X, int64_t M, int64_t N, const void* out, int64_t ld) {
     if (ld % 4 != 0) return false;
@@ -525,10 +549,7 @@ void apply_whitening_tc(const float* X, int64_t M, int64_t N, const double* W, d
     if (!ext_err) MS3_CUDA(cudaMemsetAsync(err, 0, sizeof(int), stream));
     w_split_tf32<<<(unsigned)ceil_div(M * M, 256), 256, 0, stream>>>(W, M * M, whi, wlo);
     MS3_LAUNCH_CHECK();
-    if (drain)
-        launch_apply_tc<128, true>(X, M, N, ld, whi, wlo, quantization_unit, round_1e4 ? 1 : 0, out, err, stream);
-    else
-        launch_apply_tc<128, false>(X, M, N, ld, whi, wlo, quantization_unit, round_1e4 ? 1 : 0, out, err, stream);
+    apply_tc_launch(X, M, N, ld, whi, wlo, quantization_unit, drain, round_1e4, out, err, nullptr, stream);
     if (ext_err) return;  // the caller checks the flag once for many calls
     if (host_err) {  // the caller looks at it after its own synchronisation
         MS3_CUDA(cudaMemcpyAsync(host_err, err, sizeof(int), cudaMemcpyDeviceToHost, stream));

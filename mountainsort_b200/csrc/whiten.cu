@@ -1353,10 +1353,10 @@ void apply_whitening_device(const float* X, int64_t M, int64_t N, const double* 
     const char* ffma = std::getenv("MS3GPU_APPLY_FFMA");
     const bool force_ffma = ffma && ffma[0] == '1';
     if (quantization_unit <= 0 && (mixed || !force_ffma) && apply_f16_supported(X, M, N, out, ld)) {
-        apply_whitening_f16(X, M, N, W, out, stream, err, round_1e4, ld, host_err);
+        apply_whitening_f16(X, M, N, W, /*drain=*/!mixed, out, stream, err, round_1e4, ld, host_err);
         return;
     }
-    // int16 output, and float output that TMA stores cannot reach
+    // int16 output, and float output of many channels or that TMA stores cannot reach
     if (apply_tc_supported(X, M, N, out, ld) && (mixed || !force_ffma)) {
         apply_whitening_tc(X, M, N, W, quantization_unit, /*drain=*/!mixed, out, stream, err, round_1e4, ld, host_err);
         return;

@@ -87,8 +87,9 @@ void whitening_matrix_device(const double* XXt, int64_t M, double* W, double* co
 
 // out = quantize(W^T x) per timepoint; out float32, or int16 when
 // quantization_unit > 0.  Float output on the tensor cores from 11-bit halves where
-// apply_f16_supported; otherwise three TF32 products, drained per K-block or, mixed,
-// accumulated over K, where apply_tc_supported; otherwise FP32 FMA.
+// apply_f16_supported and W's weights span less than 2^30; otherwise three TF32 products,
+// drained per K-block or, mixed, accumulated over K, where apply_tc_supported; otherwise
+// FP32 FMA.
 // err: optional device flag raised by a timed-out tensor-core pipeline; when
 // null the call keeps one of its own and copies it to host_err on the stream, or,
 // when that is null too, checks it itself (synchronising the stream).
@@ -108,10 +109,17 @@ void apply_whitening_tc(const float* X, int64_t M, int64_t N, const double* W, d
                         bool drain, void* out, cudaStream_t stream, int* err, bool round_1e4, int64_t ld,
                         int* host_err);
 
+// The kernel alone, from W's halves ([M][M], K-major).  only_if: optional device flag; the
+// kernel returns at once where it is 0.
+void apply_tc_launch(const float* X, int64_t M, int64_t N, int64_t ld, const float* whi, const float* wlo,
+                     double quantization_unit, bool drain, bool round_1e4, void* out, int* err, const int* only_if,
+                     cudaStream_t stream);
+
 // Tensor-core apply with float output from halves of 11 bits (three products,
-// round-to-nearest sums per 64 channels): both precision forms.
+// round-to-nearest sums per 64 channels): both precision forms, for a W whose weights
+// allow it (apply_f16.cu); any other W goes through apply_tc_launch, drained or not.
 bool apply_f16_supported(const float* X, int64_t M, int64_t N, const void* out, int64_t ld);
-void apply_whitening_f16(const float* X, int64_t M, int64_t N, const double* W, void* out, cudaStream_t stream,
-                         int* err, bool round_1e4, int64_t ld, int* host_err);
+void apply_whitening_f16(const float* X, int64_t M, int64_t N, const double* W, bool drain, void* out,
+                         cudaStream_t stream, int* err, bool round_1e4, int64_t ld, int* host_err);
 
 }  // namespace ms3gpu

@@ -22,3 +22,64 @@ def test_shared_memory_of_every_tiling(gpu_lib, M, precision):
     y = api.whiten_clips(X.reshape(1, N, M), W, precision=precision).reshape(N, M)
     size = X.double().abs() @ W.abs()
     assert ((y - X.double() @ W).abs() / size).max() <= BOUND
+
+
+def _bound(M, precision):
+    """Of sum |x| |w|: the TF32 form's representation, 2^-22 three times, and its truncated
+    additions, twelve to a K-block of 32 or, mixed, three to each 8 channels."""
+    return 3 * 2.0 ** -22 + (12 if precision == "plain" else 3 * -(-M // 8)) * 2.0 ** -23
+
+
+def _matrix(kind, M, g):
+    dense = 0.1 * torch.randn((M, M), generator=g, device="cuda", dtype=torch.float64) + torch.eye(M, device="cuda", dtype=torch.float64)
+    if kind == "identity":
+        return torch.eye(M, device="cuda", dtype=torch.float64)
+    if kind == "blocks":
+        b = torch.arange(M, device="cuda") // 8
+        return dense * (b[:, None] == b[None, :])
+    if kind == "tiny":
+        return torch.eye(M, device="cuda", dtype=torch.float64) + 1e-9 * dense
+    if kind == "wide":
+        return dense * 2.0 ** (-34 * torch.rand((M, M), generator=g, device="cuda", dtype=torch.float64))
+    if kind == "near":  # within the range of the 11-bit halves
+        return torch.exp2(-28.5 * torch.rand((M, M), generator=g, device="cuda", dtype=torch.float64)) + torch.eye(M, device="cuda")
+    if kind == "silent":  # no weight leads from channel 5
+        dense[5], dense[:, 5] = 0, 0
+    return dense
+
+
+@pytest.mark.parametrize("kind", ["identity", "blocks", "tiny", "wide", "near", "silent"])
+@pytest.mark.parametrize("M", [8, 96, 200, 580])
+@pytest.mark.parametrize("gain", [1.0, 1e6, 1e12])
+def test_one_loud_channel(gpu_lib, kind, M, gain):
+    """Each output is as exact as the terms that it sums, whatever a channel that hardly or
+    not at all contributes to it holds."""
+    N = 300
+    g = torch.Generator(device="cuda").manual_seed(M)
+    W = _matrix(kind, M, g)
+    X = torch.randn((N, M), generator=g, device="cuda")
+    X[:, 5] *= gain
+    ref, size = X.double() @ W, X.double().abs() @ W.abs()
+    for precision in ("plain", "mixed"):
+        y = api.whiten_clips(X.reshape(1, N, M), W, precision=precision).reshape(N, M)
+        assert ((y - ref).abs() <= _bound(M, precision) * size).all()
+
+
+@pytest.mark.parametrize("M", [8, 96, 200, 2820])
+@pytest.mark.parametrize("N", [1, 300])
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("kind", ["dense", "blocks"])
+def test_tf32_float_output(gpu_lib, M, N, offset, kind):
+    """The TF32 kernel's float output, through TMA stores (offset 0: a block matrix, or more
+    than 2816 channels) and straight from registers (off a 16-byte boundary)."""
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    W = _matrix(kind, M, g)
+    X = torch.randn((N, M), generator=g, device="cuda")
+    ref, size = X.double() @ W, X.double().abs() @ W.abs()
+    for precision in ("plain", "mixed"):
+        room = torch.full((N * M + 8,), 7.0, device="cuda")
+        out = room[offset:offset + N * M].view(N, M)
+        y = api.apply_whitening_matrix(X, W, out=out, precision=precision)
+        # the 1e-4 rounding, and its product's to a float
+        assert ((y - ref).abs() <= _bound(M, precision) * size + 5e-5 + 2.0 ** -24 * ref.abs() + 1e-9).all()
+        assert (room[:offset] == 7).all() and (room[offset + N * M:] == 7).all()
