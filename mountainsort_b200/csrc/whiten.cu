@@ -592,10 +592,12 @@ __device__ __forceinline__ void row_elements(const double (&v)[N], int base, dou
 
 __host__ __device__ constexpr int pow2_at_least(int n) { return n <= 1 ? 1 : 2 * pow2_at_least((n + 1) / 2); }
 
-template <int CS, int NW, int CPL>
+// GIVE_UP (testing): the second warp of each cluster's first CTA takes its wait of step
+// give_up_step as run out.
+template <int CS, int NW, int CPL, bool GIVE_UP = false>
 __global__ void __launch_bounds__(NW * 32, 1) pca_reg(const double* __restrict__ XXt_all, int M, int num_iter,
                                                       double* __restrict__ comps_all,
-                                                      double* __restrict__ sigma_all) {
+                                                      double* __restrict__ sigma_all, int give_up_step) {
     constexpr int G = CS * NW;             // rows per row slot of the whole cluster
     constexpr int RPW = 32 * CPL / G;      // row slots of a warp
     static_assert(RPW * G == 32 * CPL, "the rows fill the column range");
@@ -621,6 +623,7 @@ __global__ void __launch_bounds__(NW * 32, 1) pca_reg(const double* __restrict__
     __shared__ double stage[2][CS > 1 ? R : 1];  // CS > 1: this CTA's rows on their way out
     __shared__ double vinit[kMaxM];
     __shared__ __align__(8) uint64_t ybar[2];  // CS > 1: bytes of ybuf[b] received in the current step
+    __shared__ int gave_up[2];                 // CS > 1: a warp gave up in the step before (by step parity)
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
     const int base = w * CS + rank;  // row of slot 0
     const uint32_t step_bytes = (uint32_t)M * 8u;
@@ -635,6 +638,7 @@ __global__ void __launch_bounds__(NW * 32, 1) pca_reg(const double* __restrict__
         }
     for (int n = threadIdx.x; n < 2 * kYLen; n += NW * 32) (&ybuf[0][0])[n] = 0.0;
     if (CS > 1 && threadIdx.x == 0) {
+        gave_up[0] = gave_up[1] = 0;
         tc::mbar_init(&ybar[0], 1);
         tc::mbar_init(&ybar[1], 1);
         tc::fence_mbar_init();
@@ -691,7 +695,15 @@ __global__ void __launch_bounds__(NW * 32, 1) pca_reg(const double* __restrict__
     const int y0 = CS > 1 ? (l % CS) * RS + l / CS : l;
     constexpr int kYStep = CS > 1 ? 32 / CS : 32;
 
-    // ybuf[step & 1] = A v in every CTA; returns once it is complete
+    // ybuf[step & 1] = A v in every CTA; returns once it is complete.  A warp whose wait
+    // gives up leaves the loop, says so in gave_up and takes part in one more block barrier,
+    // the next step's; after that barrier the CTA's other warps see it and leave too, so
+    // that none stands in the cluster barrier while another waits for it in a block barrier.
+    // Two words by step parity: a warp that gives up in step s writes the word of s + 1; the
+    // next to write that word has passed the barrier of s + 2, which every warp reaches
+    // after its read in s + 1.  (A vote in the block barrier, __syncthreads_and, cost 180 ns
+    // a step, and so did a return of its own for a warp that sees the word: 4136 and 4903 us
+    // at 384 channels.)
     auto matvec = [&](int step) -> bool {
         const int b = step & 1;
         double s[RP2];
@@ -720,13 +732,15 @@ __global__ void __launch_bounds__(NW * 32, 1) pca_reg(const double* __restrict__
         }
         if (holds) stage[b][slot * NW + w] = s[0];
         __syncthreads();
+        const int leave = *const_cast<volatile int*>(&gave_up[b]);
         if (sends) {
             const uint64_t x = (uint64_t)__double_as_longlong(stage[b][l]);
 #pragma unroll
             for (int i = 0; i < kSends; i++)
                 tc::st_async_b64(rbuf[i] + (uint32_t)(b * kYLen * 8), x, rbar[i] + (uint32_t)(b * 8));
         }
-        const bool ok = __all_sync(0xffffffffu, tc::mbar_wait_cluster_spin(&ybar[b], (uint32_t)((step >> 1) & 1), err));
+        bool ok = __all_sync(0xffffffffu, !leave && tc::mbar_wait_cluster_spin(&ybar[b], (uint32_t)((step >> 1) & 1), err));
+        if (GIVE_UP && step == give_up_step && rank == 0 && w == 1) ok = false;  // as if it had run out
         // re-arm for step + 2: its stores arrive only after this CTA has sent step + 1
         if (ok && threadIdx.x == 0) tc::mbar_expect_tx(&ybar[b], step_bytes);
         return ok;
@@ -789,8 +803,25 @@ __global__ void __launch_bounds__(NW * 32, 1) pca_reg(const double* __restrict__
             }
         }
     }
-    // no CTA leaves while a peer may still store into its shared memory
-    if (CS > 1) cluster.sync();
+    // No CTA leaves while a peer may still store into its shared memory.  A CTA that has
+    // received every step has nothing more on its way; one that gave up lets the stores
+    // land that its peers issued before they came here.
+    if (CS > 1) {
+        // a warp that saw the word has passed the barrier that the others wait for here
+        const bool saw = !ok && *const_cast<volatile int*>(&gave_up[step & 1]);
+        if (!saw) {
+            if (!ok && l == 0) {
+                gave_up[(step & 1) ^ 1] = 1;
+                atomicExch(err, 1);
+            }
+            __syncthreads();
+        }
+        cluster.sync();
+        if (gave_up[0] || gave_up[1]) {
+            const unsigned long long t0 = tc::globaltimer_ns();
+            while (tc::globaltimer_ns() - t0 < 1000000ull) __nanosleep(1000);
+        }
+    }
 }
 
 // W = (C D) C^T, D = diag(1/sqrt(sigma)) (0 where sigma == 0), in the
@@ -1181,9 +1212,10 @@ namespace {
 
 // pca_reg for `count` matrices, one cluster each; false when the device cannot
 // hold a cluster of that size.
-template <int CS, int NW, int CPL>
-bool launch_pca_reg(const double* XXt, int64_t M, int count, double* comps, double* sigma, cudaStream_t stream) {
-    auto kern = pca_reg<CS, NW, CPL>;
+template <int CS, int NW, int CPL, bool GIVE_UP = false>
+bool launch_pca_reg(const double* XXt, int64_t M, int count, double* comps, double* sigma, cudaStream_t stream,
+                    int give_up_step = -1) {
+    auto kern = pca_reg<CS, NW, CPL, GIVE_UP>;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(CS * count), 1, 1);
     cfg.blockDim = dim3(NW * 32, 1, 1);
@@ -1204,7 +1236,7 @@ bool launch_pca_reg(const double* XXt, int64_t M, int count, double* comps, doub
         }
         if (clusters < 1) return false;
     }
-    MS3_CUDA(cudaLaunchKernelEx(&cfg, kern, XXt, (int)M, 10, comps, sigma));
+    MS3_CUDA(cudaLaunchKernelEx(&cfg, kern, XXt, (int)M, 10, comps, sigma, give_up_step));
     MS3_LAUNCH_CHECK();
     return true;
 }
@@ -1214,6 +1246,10 @@ bool launch_pca_reg(const double* XXt, int64_t M, int count, double* comps, doub
 // 0.80 us a step in one CTA, 1.04 in a cluster of eight); beyond, 16 CTAs hold it.
 // The smallest instance whose column range covers M.
 bool pca_registers(const double* XXt, int64_t M, int count, double* comps, double* sigma, cudaStream_t stream) {
+    if (const char* give_up = std::getenv("MS3GPU_PCA_GIVE_UP_STEP")) {  // testing: one size per CTA width
+        if (M > 192 && M <= 256) return launch_pca_reg<16, 4, 8, true>(XXt, M, count, comps, sigma, stream, std::atoi(give_up));
+        if (M > 384 && M <= 512) return launch_pca_reg<16, 8, 16, true>(XXt, M, count, comps, sigma, stream, std::atoi(give_up));
+    }
     if (M <= 32) return launch_pca_reg<1, 4, 1>(XXt, M, count, comps, sigma, stream);
     if (M <= 64) return launch_pca_reg<1, 8, 2>(XXt, M, count, comps, sigma, stream);
     if (M <= 96) return launch_pca_reg<1, 8, 3>(XXt, M, count, comps, sigma, stream);
