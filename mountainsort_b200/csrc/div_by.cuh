@@ -8,8 +8,8 @@
 // rounding error, is within one ulp for every mantissa.  One reciprocal serves
 // all values: four FMA-pipe operations per value instead of a division of its
 // own.  The remainder is exact and nothing overflows while |y| and |b| lie within
-// [2^-500, 2^500); other values (zeros, infinities and NaN among them) are
-// divided with the ordinary operator.
+// [2^-500, 2^500), and for y = +0 every operation gives +0.  Other values (-0,
+// infinities and NaN among them) are divided with the ordinary operator.
 #pragma once
 
 #include <cmath>
@@ -48,7 +48,7 @@ __host__ __device__ inline Reciprocal reciprocal_of(double b) {
     return c;
 }
 
-// y / b for |y| and |b| in range
+// y / b for |y| and |b| in range, or y = +0 and b > 0 in range
 __host__ __device__ inline double quotient_in_range(double y, double b, const Reciprocal& c) {
 #ifdef __CUDA_ARCH__
     const double q = __fma_rn(y, c.r, __dmul_rn(y, c.rl));

@@ -539,12 +539,14 @@ __device__ __noinline__ double plain_quotient(double y, double b) { return y / b
 
 // Whether v[j] / b may use quotient_in_range for every element with 32 j < left
 // (the others are zero and stay so), as far as v decides it; called by all lanes
-// of a warp.
+// of a warp.  +0 may: a silent channel's entry is zero in every vector (384 channels, one
+// silent: 9520 us with ordinary divisions, now 4190).
 template <int N>
 __device__ __forceinline__ bool quotients_in_range(const double (&v)[N], int left) {
     bool fast = true;
 #pragma unroll
-    for (int j = 0; j < N; j++) fast &= quotient_range(v[j]) || 32 * j >= left;
+    for (int j = 0; j < N; j++)
+        fast &= quotient_range(v[j]) || (__double2hiint(v[j]) | __double2loint(v[j])) == 0 || 32 * j >= left;
     return __all_sync(0xffffffffu, fast);
 }
 
