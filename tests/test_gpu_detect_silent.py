@@ -1,0 +1,54 @@
+"""The detector's statistics with silent channels and silent stretches: event times
+equal the oracle's, and one silent channel costs hardly more than none."""
+import numpy as np
+import pytest
+import torch
+
+from mountainsort_b200 import api
+
+pytestmark = pytest.mark.gpu
+
+
+def _data(kind, N, M):
+    rng = np.random.default_rng(N + M)
+    X = rng.standard_normal((N, M)).astype(np.float32)
+    X[:, M // 2] = 0.0  # silent throughout
+    X[: N // 2, 0] = -0.0  # silent in the first half
+    X[N // 3:, M - 1] = 0.0
+    if kind == "all":
+        X[:] = 0.0
+    if kind == "nan":
+        X[N // 2, 0] = np.nan
+        X[N // 4, M - 1] = -np.inf
+    return X
+
+
+@pytest.mark.parametrize("kind", ["some", "all", "nan"])
+@pytest.mark.parametrize("N,M,chunk", [(40000, 3, 0), (6301, 65, 100)])
+def test_event_times_equal_the_oracles(gpu_lib, ref32, kind, N, M, chunk):
+    X = _data(kind, N, M)
+    for thr, interval, sign in ((2.0, 25.5, -1), (0.0, 10.0, 0)):
+        got = api.detect_events(X, detect_threshold=thr, detect_interval=interval, detect_sign=sign, chunk_size=chunk)
+        ref = ref32.detect_events(X, detect_threshold=thr, detect_interval=interval, detect_sign=sign,
+                                  chunk_size=chunk or None)
+        for m in range(M):
+            np.testing.assert_array_equal(got[m], ref[m])
+
+
+def test_time_with_a_silent_channel(gpu_lib):
+    def ms(X):
+        best = 1e9
+        for _ in range(4):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            api.detect_events(X, detect_threshold=5.0, detect_interval=30.0, detect_sign=-1)
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b))
+        return best
+
+    g = torch.Generator(device="cuda").manual_seed(1)
+    X = torch.round(torch.randn((1_000_000, 64), generator=g, device="cuda") * 1e4) / 1e4
+    plain = ms(X)
+    X[:, 20] = 0.0
+    assert ms(X) <= 2 * plain  # sample by sample: 20 times
