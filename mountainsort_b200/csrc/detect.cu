@@ -19,7 +19,8 @@
 //
 // The index-order sums are what a long recording waits for if one thread forms
 // them (two dependent FP64 additions per sample: 59 ms for 64 channels x 1.8M,
-// one chunk).  They are formed in parallel with the same bits:
+// one chunk).  With thousands of (channel, chunk) pairs a thread does (serial_stats);
+// fewer are formed in parallel with the same bits:
 //   sum of x    When every partial sum is a multiple of 2^q and at most
 //               2^(53 + q) in magnitude, no addition rounds and any order gives
 //               the value.  2^q divides the samples (floats) and the sum so far;
@@ -147,6 +148,23 @@ __device__ __forceinline__ ChunkStats stats_of(double sum, double sumsqr, int64_
     const double stdev =
         len >= 2 ? sqrt(__ddiv_rn(__dsub_rn(sumsqr, __ddiv_rn(__dmul_rn(sum, sum), ct)), ct - 1.0)) : 0.0;
     return {mean, __dmul_rn(detect_threshold, stdev)};
+}
+
+// The statistics of one (channel, chunk) per thread, sample by sample: where there are
+// enough of them to fill the GPU (serial_stats).
+__global__ void __launch_bounds__(32) detect_stats_serial(const float* __restrict__ X, Dims d, double detect_threshold,
+                                                          ChunkStats* __restrict__ stats) {
+    const int64_t i = (int64_t)blockIdx.x * 32 + threadIdx.x;
+    if (i >= d.M * d.nchunks) return;
+    const int64_t c = i / d.M, m = i - c * d.M;
+    const int64_t len = chunk_size_at(c, d.chunk, d.N) + 2 * d.pad;
+    double sum = 0.0, sumsqr = 0.0;
+    for_samples<32>(X, d, m, c, 0, len, [&](int64_t, float x) {
+        const double v = (double)x;
+        sum = __dadd_rn(sum, v);
+        sumsqr = __dadd_rn(sumsqr, __dmul_rn(v, v));
+    });
+    stats[i] = stats_of(sum, sumsqr, len, detect_threshold);
 }
 
 __device__ __forceinline__ int binade_of(double x) {  // floor(log2 x) for normal x > 0
@@ -518,6 +536,18 @@ void prefix_sums(const T* in, int64_t n, int64_t* out, cudaStream_t stream) {
     MS3_LAUNCH_CHECK();
 }
 
+// Whether a thread per (channel, chunk) forms the statistics.  From 4096 pairs on they
+// hide one another's additions, and the segments' passes over X and the segments that go
+// sample by sample cost more.  Whole calls, us, serial and by segments:
+//   pairs (chunk)                 rounded to 1e-4   unrounded   values over 40 octaves
+//    3840 (64 ch,  30 k)           1277    984      1263   1415      2459   3294
+//    5376 (384 ch, 30 k)           1545   1444      1554   1798      3163   4667
+//    6144 (1536 ch, 163 k)         7065   5810      7063   8066     20018  27686
+//    7680 (128 ch, 30 k)           1475   1608      1467   2030      3746   5735
+//   30720 (1536 ch, 30 k)          3690   6476      3670   6915     16579  26455
+// and 1536 (384 ch, 651 k): 19639 and 4236, 19643 and 11706, 29235 and 26311.
+bool serial_stats(int64_t pairs) { return pairs >= 4096; }
+
 }  // namespace
 
 int64_t detect_chunk_size(int64_t M, int64_t N, int64_t num_simultaneous) {
@@ -544,7 +574,10 @@ void detect_events_device(const float* X, int64_t M, int64_t N, double detect_th
     const dim3 gs((unsigned)work_blocks, (unsigned)nchunks);
 
     DevBuf stats(sizeof(ChunkStats) * (size_t)MC, stream);
-    {
+    if (serial_stats(MC)) {
+        detect_stats_serial<<<(unsigned)ceil_div(MC, 32), 32, 0, stream>>>(X, d, detect_threshold, stats.as<ChunkStats>());
+        MS3_LAUNCH_CHECK();
+    } else {
         DevBuf sx(sizeof(double) * (size_t)slots, stream), sa(sizeof(float) * (size_t)slots, stream),
             sq(sizeof(double) * (size_t)slots, stream), sm(sizeof(uint32_t) * (size_t)slots, stream),
             se(sizeof(int) * (size_t)slots, stream), i0(sizeof(int64_t) * (size_t)slots, stream),
