@@ -27,6 +27,7 @@
 #include "ms3gpu.h"
 #include "pipeline.h"
 #include "ptrkind.h"
+#include "timeouts.h"
 #include "stream.h"
 #include "whiten.h"
 
@@ -225,10 +226,10 @@ public:
     void finish() {
         MS3_CUDA(cudaStreamSynchronize(s_));
         pending_ = false;
-        if (w_[3]) throw Error(MS3GPU_ERR_CUDA, "tensor-core apply: pipeline wait timed out");
-        bandpass_raise_timeout(w_[0], s_);
-        covariance_raise_timeout(w_[1], s_);
-        whitening_raise_timeout(w_[2], s_);
+        raise_together<Error>(
+            [&] { if (w_[3]) throw Error(MS3GPU_ERR_CUDA, "tensor-core apply: pipeline wait timed out"); },
+            [&] { bandpass_raise_timeout(w_[0], s_); }, [&] { covariance_raise_timeout(w_[1], s_); },
+            [&] { whitening_raise_timeout(w_[2], s_); });
     }
 
 private:
@@ -611,8 +612,7 @@ int ms3gpu_bandpass_whiten_batch(ms3gpu_job* jobs, int32_t n_jobs, void* stream)
         }
         MS3_CUDA(cudaEventDestroy(start));
         if (large_done) MS3_CUDA(cudaEventDestroy(large_done));
-        bandpass_check_timeout(s0);
-        covariance_check_timeout(s0);
+        raise_together<Error>([&] { bandpass_check_timeout(s0); }, [&] { covariance_check_timeout(s0); });
     });
     if (rc != MS3GPU_OK) return rc;
     if (first_code != MS3GPU_OK) {

@@ -72,6 +72,7 @@
 #include "cov_share.h"
 #include "ms3gpu.h"
 #include "tc_sm100.cuh"
+#include "timeouts.h"
 #include "whiten.h"
 
 namespace ms3gpu {
@@ -698,8 +699,7 @@ void covariance_check_timeout(cudaStream_t stream) {
     int h = 0;
     covariance_read_timeout(&h, stream);
     MS3_CUDA(cudaStreamSynchronize(stream));
-    covariance_raise_timeout(h, stream);
-    whitening_check_timeout(stream);
+    raise_together<Error>([&] { covariance_raise_timeout(h, stream); }, [&] { whitening_check_timeout(stream); });
 }
 
 void covariance_raise_timeout(int flag, cudaStream_t stream) {

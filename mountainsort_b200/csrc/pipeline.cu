@@ -19,6 +19,7 @@
 #include "common.cuh"
 #include "ms3gpu.h"
 #include "pipeline.h"
+#include "timeouts.h"
 #include "whiten.h"
 
 namespace ms3gpu {
@@ -163,9 +164,9 @@ void bandpass_whiten_streamed(const float* raw_h, int64_t M, int64_t N, float* f
     int herr = 0;
     MS3_CUDA(cudaMemcpyAsync(&herr, errbuf.get(), sizeof(int), cudaMemcpyDeviceToHost, s));
     MS3_CUDA(cudaStreamSynchronize(s));
-    if (herr) throw Error(MS3GPU_ERR_CUDA, "tensor-core apply: pipeline wait timed out");
-    bandpass_check_timeout(s);
-    covariance_check_timeout(s);
+    raise_together<Error>(
+        [&] { if (herr) throw Error(MS3GPU_ERR_CUDA, "tensor-core apply: pipeline wait timed out"); },
+        [&] { bandpass_check_timeout(s); }, [&] { covariance_check_timeout(s); });
 }
 
 }  // namespace ms3gpu
