@@ -1284,8 +1284,12 @@ void whitening_matrix_device(const double* XXt, int64_t M, double* W, double* co
         for (int64_t k = 0; k < count; k++)
             pca_launch_smem(XXt + k * M * M, M, comps + k * M * M, sigma + k * M, stream);
     const unsigned wt = (unsigned)ceil_div(M, kWT);
-    w_assemble<<<dim3(wt, wt, (unsigned)count), 256, 0, stream>>>(comps, sigma, (int)M, W);
-    MS3_LAUNCH_CHECK();
+    constexpr int kMaxZ = 65535;  // matrices of one launch
+    for (int k = 0; k < count; k += kMaxZ) {
+        w_assemble<<<dim3(wt, wt, (unsigned)std::min(count - k, kMaxZ)), 256, 0, stream>>>(
+            comps + k * M * M, sigma + k * M, (int)M, W + k * M * M);
+        MS3_LAUNCH_CHECK();
+    }
 }
 
 void whitening_read_timeout(int* flag, cudaStream_t stream) {
