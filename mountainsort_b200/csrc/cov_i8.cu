@@ -69,6 +69,7 @@
 #include <string>
 
 #include "common.cuh"
+#include "cov_ring.h"
 #include "cov_share.h"
 #include "ms3gpu.h"
 #include "tc_sm100.cuh"
@@ -92,7 +93,7 @@ constexpr int kPlaneStage = 2 * 4 * kPlaneBytes;
 constexpr int kConvWarps = 16;
 constexpr int kThreads = (2 + kConvWarps + 4) * 32;  // 704
 static_assert(kKT == 2 * kConvWarps, "each thread of a group of half the converter warps takes four rows of a stage");
-static_assert(kS1 == kS2, "the converters walk both rings with one stage counter");
+static_assert(kS1 == kS2 && kS1 % 2 == 1, "the converters walk both rings with one stage counter (cov_ring.h)");
 constexpr int kSentinel = 1000;               // scale exponent of a channel whose run holds inf / NaN
 constexpr size_t kSmemBytes = (size_t)kS1 * kF32Stage + (size_t)kS2 * kPlaneStage + 2 * kB * sizeof(int) +
                               1024 /*align*/ + 256 /*barriers*/;
@@ -467,8 +468,9 @@ __global__ void __launch_bounds__(kThreads, 1)
                     gph ^= 1u;
                 }
                 if ((int)(g & 1) != grp) continue;
-                ok = tc::mbar_wait(&f_full[s1], ph, err);
-                if (ok && g >= kS2) ok = tc::mbar_wait(&p_empty[s2], ph ^ 1u, err);
+                ok = converter_may_take(
+                    g, kS2, ph, [&](uint32_t p) { return tc::mbar_wait(&p_empty[s2], p, err); },
+                    [&](uint32_t p) { return tc::mbar_wait(&f_full[s1], p, err); });
                 if (!__all_sync(0xffffffffu, ok)) {
                     ok = false;
                     break;
