@@ -488,59 +488,76 @@ struct SplitW {
     int *wide, *err;        // err: null, or cleared
 };
 
-// Column m of W^T divided by the channels' scales, one warp: E = floor(log2 max), the
+// Column m of W^T divided by the channels' scales, WARPS warps: E = floor(log2 max), the
 // column's scale 2^E, the column times 2^(14 - E) as halves w_h = rn(w), w_l = rn((w -
 // w_h) 2^11), Kp of them (zeros beyond M).  A column with magnitudes beyond the float
 // range, infinities or NaN gets the scale NaN.  *wide is set for a weight below 2^-30 of
 // the column's largest or of its K-block's root sum of squares.
+// The warps take the K-blocks in turn.  (One warp a column took 13.5 us at 384 channels,
+// a third of the time of a call with few timepoints.)
+template <int WARPS>
 __device__ __forceinline__ void split_column(const double* __restrict__ w, int64_t m, int64_t M, int64_t Kp,
                                              const float* in_scale, const SplitW& o) {
-    const int l = threadIdx.x & 31;
-    double top = 0.0;
-    bool finite = true;
-#pragma unroll 4
-    for (int64_t k = l; k < M; k += 32) {
-        finite &= fabs(w[k]) < 0x1p128;
-        top = fmax(top, finite_abs(w[k]) * inverse_pow2(in_scale[k]));
-    }
-    for (int o = 16; o > 0; o >>= 1) top = fmax(top, __shfl_xor_sync(0xffffffffu, top, o));
-    finite = __all_sync(0xffffffffu, finite);
-    const int e = exponent_of(top);
-    const double s = __hiloint2double((1023 + 14 - e) << 20, 0);
-    bool small = false;
-    for (int64_t k0 = 0; k0 < M; k0 += kKB) {
-        double a2[2] = {0.0, 0.0};
-        bool counts[2];
+    const int l = threadIdx.x & 31, first = WARPS > 1 ? threadIdx.x >> 5 : 0;
+    double top = 0.0, least = 1e300;  // of the magnitudes; of their squares
+    bool finite = true, narrow = true;
+#pragma unroll 2
+    for (int64_t k0 = first * kKB; k0 < M; k0 += WARPS * kKB) {
+        double sum = 0.0, low = 1e300;
 #pragma unroll
         for (int i = 0; i < 2; i++) {
             const int64_t k = k0 + l + 32 * i;
-            counts[i] = k < M && in_scale[k] != 0.f;
-            if (counts[i]) {
-                const double a = finite_abs(w[k]) * inverse_pow2(in_scale[k]);
-                a2[i] = a * a;
-            }
+            const double v = k < M ? w[k] : 0.0;
+            const float scale = k < M ? in_scale[k] : 0.f;
+            finite &= fabs(v) < 0x1p128;
+            const double a = finite_abs(v) * inverse_pow2(scale);
+            top = fmax(top, a);
+            sum += a * a;
+            if (scale != 0.f) low = fmin(low, a * a);
         }
-        double sum = a2[0] + a2[1];
-        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        const double least = 0x1p-60 * fmax(sum, top * top);
-        small |= (counts[0] && a2[0] < least) || (counts[1] && a2[1] < least);
+        for (int s = 16; s > 0; s >>= 1) {
+            sum += __shfl_xor_sync(0xffffffffu, sum, s);
+            low = fmin(low, __shfl_xor_sync(0xffffffffu, low, s));
+        }
+        narrow &= low >= 0x1p-60 * sum;
+        least = fmin(least, low);
     }
-    if (small && finite) *o.wide = 1;
+    for (int s = 16; s > 0; s >>= 1) top = fmax(top, __shfl_xor_sync(0xffffffffu, top, s));
+    finite = __all_sync(0xffffffffu, finite);
+    if (WARPS > 1) {
+        __shared__ double tops[WARPS], leasts[WARPS];
+        if (l == 0) {
+            tops[first] = top;
+            leasts[first] = least;
+        }
+        finite = __syncthreads_and(finite);
+        narrow = __syncthreads_and(narrow);
+        for (int i = 0; i < WARPS; i++) {
+            top = fmax(top, tops[i]);
+            least = fmin(least, leasts[i]);
+        }
+    }
+    const int e = exponent_of(top);
+    if (l == 0 && first == 0) {
+        if (finite && !(narrow && least >= 0x1p-60 * (top * top))) *o.wide = 1;
+        o.col_scale[m] = finite ? pow2f(e) : __uint_as_float(0x7FC00000u);
+    }
+    const double s = __hiloint2double((1023 + 14 - e) << 20, 0);
     __half* hi = o.hi + m * Kp;
     __half* lo = o.lo + m * Kp;
 #pragma unroll 4
-    for (int64_t k = l; k < Kp; k += 32) {
-        const double x = k < M ? w[k] * inverse_pow2(in_scale[k]) * s : 0.0;
+    for (int64_t k = first * 32 + l; k < Kp; k += WARPS * 32) {
+        const double v = k < M ? w[k] : 0.0;
+        const double x = k < M ? v * inverse_pow2(in_scale[k]) * s : 0.0;
         const __half h = __double2half(x);
         hi[k] = h;
         lo[k] = __double2half((x - (double)__half2float(h)) * (double)kLowScale);
         if (k < M) {
-            const float h32 = __uint_as_float(tc::cvt_rna_tf32((float)w[k]));
+            const float h32 = __uint_as_float(tc::cvt_rna_tf32((float)v));
             o.hi32[m * M + k] = h32;
-            o.lo32[m * M + k] = __uint_as_float(tc::cvt_rna_tf32((float)(w[k] - (double)h32)));
+            o.lo32[m * M + k] = __uint_as_float(tc::cvt_rna_tf32((float)(v - (double)h32)));
         }
     }
-    if (l == 0) o.col_scale[m] = finite ? pow2f(e) : __uint_as_float(0x7FC00000u);
 }
 
 __device__ __forceinline__ float in_scale_of(double top) { return top > 0.0 ? pow2f(exponent_of(top)) : 0.f; }
@@ -555,7 +572,7 @@ __global__ void __launch_bounds__(1024) w_in_scales(const double* __restrict__ W
     const int64_t k = (int64_t)blockIdx.x * 32 + l;
     double top = 0.0;
     if (k < M) {
-#pragma unroll 4
+#pragma unroll 8
         for (int64_t m = p; m < M; m += 32) top = fmax(top, finite_abs(W[m * M + k]));
     }
     part[p][l] = top;
@@ -569,8 +586,8 @@ __global__ void __launch_bounds__(1024) w_in_scales(const double* __restrict__ W
 
 __global__ void __launch_bounds__(128) w_split_f16(const double* __restrict__ W, int64_t M, int64_t Kp, SplitW o) {
     if (o.err && blockIdx.x == 0 && threadIdx.x == 0) *o.err = 0;
-    const int64_t m = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
-    if (m < M) split_column(W + m * M, m, M, Kp, o.in_scale, o);
+    const int64_t m = blockIdx.x;
+    split_column<4>(W + m * M, m, M, Kp, o.in_scale, o);
 }
 
 // Both in one block for up to 64 channels, where a launch costs more than the work.
@@ -603,7 +620,7 @@ __global__ void __launch_bounds__(1024) w_prepare_small(const double* __restrict
         o.in_scale[k] = scale[k] = in_scale_of(top);
     }
     __syncthreads();
-    for (int m = threadIdx.x >> 5; m < M; m += 32) split_column(copy + m * M, m, M, Kp, scale, o);
+    for (int m = threadIdx.x >> 5; m < M; m += 32) split_column<1>(copy + m * M, m, M, Kp, scale, o);
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn_f16() {
@@ -687,7 +704,7 @@ void apply_whitening_f16(const float* X, int64_t M, int64_t N, const double* W, 
     } else {
         w_in_scales<<<(unsigned)ceil_div(n_in, 32), 1024, 0, stream>>>(W, M, n_in, w);
         MS3_LAUNCH_CHECK();
-        w_split_f16<<<(unsigned)ceil_div(M, 4), 128, 0, stream>>>(W, M, Kp, w);
+        w_split_f16<<<(unsigned)M, 128, 0, stream>>>(W, M, Kp, w);
     }
     MS3_LAUNCH_CHECK();
     const CUtensorMap mx = matrix_map(CU_TENSOR_MAP_DATA_TYPE_FLOAT32, X, (uint64_t)M, (uint64_t)N,
