@@ -11,7 +11,7 @@
 //      index order (MLCompute::mean / stdev, common/mlcompute.cpp:67-85);
 //   2. the candidates -- samples whose signed (or absolute, for sign 0)
 //      deviation from the mean exceeds threshold * stdev -- counted and written
-//      in time order, a thread per (channel, segment of kSeg samples);
+//      in time order, a thread per (channel, segment of samples);
 //   3. the reference's greedy strongest-within-detect_interval rule.  Between
 //      candidates more than the interval apart it starts afresh, so a thread
 //      takes each run of closer ones;
@@ -46,6 +46,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <utility>
 #include <vector>
 
 #include "common.cuh"
@@ -55,7 +56,8 @@ namespace ms3gpu {
 
 namespace {
 
-constexpr int kSeg = 512;    // samples per segment
+constexpr int kSeg = 512;    // samples per segment at most
+constexpr int kShortSeg = 64;  // where there are few of them (segment_length)
 constexpr int kBatch = 16;   // samples loaded together
 
 struct ChunkStats {
@@ -64,6 +66,7 @@ struct ChunkStats {
 
 struct Dims {
     int64_t M, N, chunk, pad, nchunks, nseg;  // nseg: segments of the longest chunk
+    int seg;                                  // samples per segment
 };
 
 __device__ __forceinline__ int64_t chunk_size_at(int64_t c, int64_t chunk, int64_t N) {
@@ -111,8 +114,8 @@ __device__ __forceinline__ Work segment_work(const Dims& d) {
     w.m = i - w.s * d.M;
     w.c = blockIdx.y;
     const int64_t len = chunk_size_at(w.c, d.chunk, d.N) + 2 * d.pad;
-    w.a = w.s * kSeg;
-    w.e = w.a + kSeg < len ? w.a + kSeg : len;
+    w.a = w.s * d.seg;
+    w.e = w.a + d.seg < len ? w.a + d.seg : len;
     w.any = w.s < d.nseg;
     w.slot = (w.m * d.nchunks + w.c) * d.nseg + w.s;
     return w;
@@ -251,6 +254,7 @@ __device__ __forceinline__ bool sums_exact(double bound, int q) {
 
 // The reference's statistics of one (channel, chunk) per warp.
 constexpr int kStatWarps = 2;
+template <int SEG>  // d.seg
 __global__ void __launch_bounds__(32 * kStatWarps) detect_stats(const float* __restrict__ X, Dims d,
                                                                double detect_threshold,
                                                                const double* __restrict__ seg_x,
@@ -260,7 +264,7 @@ __global__ void __launch_bounds__(32 * kStatWarps) detect_stats(const float* __r
                                                                const int64_t* __restrict__ seg_inc0,
                                                                const int64_t* __restrict__ seg_inc1,
                                                                ChunkStats* __restrict__ stats) {
-    __shared__ __align__(16) float staged[kStatWarps][kSeg];
+    __shared__ __align__(16) float staged[kStatWarps][SEG];
     const int l = threadIdx.x & 31;
     const int64_t k = (int64_t)blockIdx.x * kStatWarps + (threadIdx.x >> 5);
     if (k >= d.M * d.nchunks) return;
@@ -268,14 +272,14 @@ __global__ void __launch_bounds__(32 * kStatWarps) detect_stats(const float* __r
     const int64_t m = k / d.nchunks, c = k - m * d.nchunks;
     const int64_t t1 = c * d.chunk;
     const int64_t len = chunk_size_at(c, d.chunk, d.N) + 2 * d.pad;
-    const int64_t nseg = (len + kSeg - 1) / kSeg;
+    const int64_t nseg = (len + SEG - 1) / SEG;
     double sum = 0.0, sumsqr = 0.0;
 
     auto one_by_one = [&](int64_t s) {
-        const int64_t a = s * kSeg;
-        const int n = (int)(a + kSeg < len ? kSeg : len - a);
+        const int64_t a = s * SEG;
+        const int n = (int)(a + SEG < len ? SEG : len - a);
         __syncwarp();
-        for (int i = l; i < kSeg; i += 32) {
+        for (int i = l; i < SEG; i += 32) {
             const int64_t t = t1 - d.pad + a + i;
             mine[i] = (i < n && t >= 0 && t < d.N) ? X[t * d.M + m] : 0.f;
         }
@@ -511,8 +515,8 @@ template <class T>
 __global__ void __launch_bounds__(256) scan_write(const T* __restrict__ in, int64_t n, const int64_t* __restrict__ sums,
                                                   int64_t* __restrict__ out) {
     __shared__ int64_t red[8];
-    int64_t before = sums[blockIdx.x];
-    for (int64_t b = (int64_t)blockIdx.x * kScanItems, e = b + kScanItems; b < e; b += 256) {
+    int64_t before = sums ? sums[blockIdx.x] : 0;
+    for (int64_t b = (int64_t)blockIdx.x * kScanItems, e = b + kScanItems; b < e && b < n; b += 256) {
         const int64_t i = b + threadIdx.x;
         int64_t total;
         const int64_t v = i < n ? (int64_t)in[i] : 0;
@@ -523,18 +527,41 @@ __global__ void __launch_bounds__(256) scan_write(const T* __restrict__ in, int6
     }
 }
 
-// n >= 1
+int64_t scan_blocks(int64_t n) { return ceil_div(n, kScanItems); }
+
+// n >= 1; sums: scan_blocks(n) values
 template <class T>
-void prefix_sums(const T* in, int64_t n, int64_t* out, cudaStream_t stream) {
-    const int64_t blocks = ceil_div(n, kScanItems);
-    DevBuf sums(sizeof(int64_t) * (size_t)blocks, stream);
-    scan_block_sums<<<(unsigned)blocks, 256, 0, stream>>>(in, n, sums.as<int64_t>());
-    MS3_LAUNCH_CHECK();
-    scan_of_sums<<<1, 256, 0, stream>>>(sums.as<int64_t>(), blocks);
-    MS3_LAUNCH_CHECK();
-    scan_write<<<(unsigned)blocks, 256, 0, stream>>>(in, n, sums.as<int64_t>(), out);
+void prefix_sums(const T* in, int64_t n, int64_t* out, int64_t* sums, cudaStream_t stream) {
+    const int64_t blocks = scan_blocks(n);
+    if (blocks > 1) {
+        scan_block_sums<<<(unsigned)blocks, 256, 0, stream>>>(in, n, sums);
+        MS3_LAUNCH_CHECK();
+        scan_of_sums<<<1, 256, 0, stream>>>(sums, blocks);
+        MS3_LAUNCH_CHECK();
+    }
+    scan_write<<<(unsigned)blocks, 256, 0, stream>>>(in, n, blocks > 1 ? sums : nullptr, out);
     MS3_LAUNCH_CHECK();
 }
+
+// Arrays of one allocation: short recordings waited for the allocations and frees of one
+// each (1 channel x 100 timepoints: 292 us a call, with one allocation 259).
+class Arrays {
+public:
+    template <class T>
+    void add(T** p, int64_t n) {
+        parts_.push_back({reinterpret_cast<void**>(p), bytes_});
+        bytes_ += (sizeof(T) * (size_t)n + 255) / 256 * 256;
+    }
+    void alloc(cudaStream_t stream) {
+        buf_.alloc(bytes_, stream);
+        for (const auto& p : parts_) *p.first = buf_.as<char>() + p.second;
+    }
+
+private:
+    std::vector<std::pair<void**, size_t>> parts_;
+    size_t bytes_ = 0;
+    DevBuf buf_;
+};
 
 // Whether a thread per (channel, chunk) forms the statistics.  From 4096 pairs on they
 // hide one another's additions, and the segments' passes over X and the segments that go
@@ -547,6 +574,14 @@ void prefix_sums(const T* in, int64_t n, int64_t* out, cudaStream_t stream) {
 //   30720 (1536 ch, 30 k)          3690   6476      3670   6915     16579  26455
 // and 1536 (384 ch, 651 k): 19639 and 4236, 19643 and 11706, 29235 and 26311.
 bool serial_stats(int64_t pairs) { return pairs >= 4096; }
+
+// A thread takes a segment, 16 loads at a time: with few threads a pass over segments of
+// 512 waits for 32 such batches one after another.  Short chunks (at most eight times 32
+// segments of 64, which detect_stats puts together one after another) with few of them
+// take 64 (1 channel x 100 timepoints: 259 and 141 us a call; 16 x 8000: 287 and 184).
+int segment_length(int64_t len, int64_t pairs) {
+    return len <= 8 * 32 * kShortSeg && pairs * ceil_div(len, kSeg) < 16384 ? kShortSeg : kSeg;
+}
 
 }  // namespace
 
@@ -566,76 +601,91 @@ void detect_events_device(const float* X, int64_t M, int64_t N, double detect_th
     if (M <= 0 || N <= 0) return;
     const int64_t nchunks = ceil_div(N, chunk);
     if (nchunks > 65535) throw_unsupported("too many time chunks");
-    Dims d{M, N, chunk, pad, nchunks, ceil_div(std::min(chunk, N) + 2 * pad, kSeg)};
+    const int64_t len = std::min(chunk, N) + 2 * pad;
+    const int seg = segment_length(len, M * nchunks);
+    Dims d{M, N, chunk, pad, nchunks, ceil_div(len, seg), seg};
     const int64_t MC = M * nchunks, slots = MC * d.nseg;
     if (MC > 0x7fffffff) throw_unsupported("too many (channel, chunk) pairs");
     const int64_t work_blocks = ceil_div(M * d.nseg, 256);
     if (work_blocks > 0x7fffffff) throw_unsupported("too many segments");
     const dim3 gs((unsigned)work_blocks, (unsigned)nchunks);
 
-    DevBuf stats(sizeof(ChunkStats) * (size_t)MC, stream);
+    ChunkStats* stats;
+    int64_t *base, *cnt, *sums;  // candidates, channel-major, then chunk, then segment (time order)
+    Arrays first;
+    first.add(&stats, MC);
+    first.add(&base, slots + 1);
+    first.add(&cnt, slots);
+    first.add(&sums, scan_blocks(slots));
+    first.alloc(stream);
     if (serial_stats(MC)) {
-        detect_stats_serial<<<(unsigned)ceil_div(MC, 32), 32, 0, stream>>>(X, d, detect_threshold, stats.as<ChunkStats>());
+        detect_stats_serial<<<(unsigned)ceil_div(MC, 32), 32, 0, stream>>>(X, d, detect_threshold, stats);
         MS3_LAUNCH_CHECK();
     } else {
-        DevBuf sx(sizeof(double) * (size_t)slots, stream), sa(sizeof(float) * (size_t)slots, stream),
-            sq(sizeof(double) * (size_t)slots, stream), sm(sizeof(uint32_t) * (size_t)slots, stream),
-            se(sizeof(int) * (size_t)slots, stream), i0(sizeof(int64_t) * (size_t)slots, stream),
-            i1(sizeof(int64_t) * (size_t)slots, stream);
-        detect_segments<<<gs, 256, 0, stream>>>(X, d, sx.as<double>(), sa.as<float>(), sq.as<double>(),
-                                                sm.as<uint32_t>());
+        double *sx, *sq;
+        float* sa;
+        uint32_t* sm;
+        int* se;
+        int64_t *i0, *i1;
+        Arrays segs;
+        segs.add(&sx, slots);
+        segs.add(&sa, slots);
+        segs.add(&sq, slots);
+        segs.add(&sm, slots);
+        segs.add(&se, slots);
+        segs.add(&i0, slots);
+        segs.add(&i1, slots);
+        segs.alloc(stream);
+        detect_segments<<<gs, 256, 0, stream>>>(X, d, sx, sa, sq, sm);
         MS3_LAUNCH_CHECK();
-        detect_binades<<<(unsigned)ceil_div(MC, 4), 128, 0, stream>>>(sq.as<double>(), MC, d.nseg, se.as<int>());
+        detect_binades<<<(unsigned)ceil_div(MC, 4), 128, 0, stream>>>(sq, MC, d.nseg, se);
         MS3_LAUNCH_CHECK();
-        detect_increments<<<gs, 256, 0, stream>>>(X, d, sq.as<double>(), se.as<int>(), i0.as<int64_t>(),
-                                                  i1.as<int64_t>());
+        detect_increments<<<gs, 256, 0, stream>>>(X, d, sq, se, i0, i1);
         MS3_LAUNCH_CHECK();
-        detect_stats<<<(unsigned)ceil_div(MC, kStatWarps), 32 * kStatWarps, 0, stream>>>(
-            X, d, detect_threshold, sx.as<double>(), sa.as<float>(), sm.as<uint32_t>(), se.as<int>(),
-            i0.as<int64_t>(), i1.as<int64_t>(), stats.as<ChunkStats>());
+        const auto stats_kernel = seg == kSeg ? detect_stats<kSeg> : detect_stats<kShortSeg>;
+        stats_kernel<<<(unsigned)ceil_div(MC, kStatWarps), 32 * kStatWarps, 0, stream>>>(X, d, detect_threshold, sx, sa, sm,
+                                                                                       se, i0, i1, stats);
         MS3_LAUNCH_CHECK();
     }
-    // candidates, channel-major, then chunk, then segment (time order)
-    DevBuf base(sizeof(int64_t) * (size_t)(slots + 1), stream);
-    {
-        DevBuf cnt(sizeof(int64_t) * (size_t)slots, stream);
-        detect_candidates<false><<<gs, 256, 0, stream>>>(X, d, stats.as<ChunkStats>(), sign, cnt.as<int64_t>(), nullptr,
-                                                         nullptr, nullptr, nullptr);
-        MS3_LAUNCH_CHECK();
-        prefix_sums(cnt.as<int64_t>(), slots, base.as<int64_t>(), stream);
-    }
+    detect_candidates<false><<<gs, 256, 0, stream>>>(X, d, stats, sign, cnt, nullptr, nullptr, nullptr, nullptr);
+    MS3_LAUNCH_CHECK();
+    prefix_sums(cnt, slots, base, sums, stream);
     int64_t ncand = 0;
-    MS3_CUDA(cudaMemcpyAsync(&ncand, base.as<int64_t>() + slots, sizeof(int64_t), cudaMemcpyDeviceToHost, stream));
+    MS3_CUDA(cudaMemcpyAsync(&ncand, base + slots, sizeof(int64_t), cudaMemcpyDeviceToHost, stream));
     MS3_CUDA(cudaStreamSynchronize(stream));
     if (ncand > ((int64_t)1 << 31)) throw_unsupported("too many threshold crossings (lower the sensitivity)");
     if (ncand == 0) return;
-    DevBuf cn(sizeof(int64_t) * (size_t)ncand, stream), cv(sizeof(double) * (size_t)ncand, stream),
-        ck(sizeof(int32_t) * (size_t)ncand, stream), use((size_t)ncand, stream),
-        at(sizeof(int64_t) * (size_t)(ncand + 1), stream), dcounts(sizeof(int64_t) * (size_t)M, stream);
-    detect_candidates<true><<<gs, 256, 0, stream>>>(X, d, stats.as<ChunkStats>(), sign, nullptr, base.as<int64_t>(),
-                                                    cn.as<int64_t>(), cv.as<double>(), ck.as<int32_t>());
+    int64_t *cn, *at, *dcounts, *dtimes, *cand_sums;
+    double* cv;
+    int32_t* ck;
+    uint8_t* use;
+    Arrays cand;
+    cand.add(&cn, ncand);
+    cand.add(&cv, ncand);
+    cand.add(&ck, ncand);
+    cand.add(&use, ncand);
+    cand.add(&at, ncand + 1);
+    cand.add(&dcounts, M);
+    cand.add(&dtimes, ncand);
+    cand.add(&cand_sums, scan_blocks(ncand));
+    cand.alloc(stream);
+    detect_candidates<true><<<gs, 256, 0, stream>>>(X, d, stats, sign, nullptr, base, cn, cv, ck);
     MS3_LAUNCH_CHECK();
     const unsigned gg = (unsigned)ceil_div(ncand, 128);
-    detect_greedy<<<gg, 128, 0, stream>>>(d, ncand, detect_interval, cn.as<int64_t>(), cv.as<double>(),
-                                          ck.as<int32_t>(), use.as<uint8_t>());
+    detect_greedy<<<gg, 128, 0, stream>>>(d, ncand, detect_interval, cn, cv, ck, use);
     MS3_LAUNCH_CHECK();
-    prefix_sums(use.as<uint8_t>(), ncand, at.as<int64_t>(), stream);
-    detect_channel_counts<<<(unsigned)ceil_div(M, 128), 128, 0, stream>>>(d, base.as<int64_t>(), at.as<int64_t>(),
-                                                                         dcounts.as<int64_t>());
+    prefix_sums(use, ncand, at, cand_sums, stream);
+    detect_channel_counts<<<(unsigned)ceil_div(M, 128), 128, 0, stream>>>(d, base, at, dcounts);
     MS3_LAUNCH_CHECK();
-    MS3_CUDA(cudaMemcpyAsync(counts.data(), dcounts.get(), sizeof(int64_t) * counts.size(), cudaMemcpyDeviceToHost,
-                             stream));
+    detect_write<<<gg, 128, 0, stream>>>(d, ncand, cn, ck, use, at, dtimes);
+    MS3_LAUNCH_CHECK();
+    MS3_CUDA(cudaMemcpyAsync(counts.data(), dcounts, sizeof(int64_t) * counts.size(), cudaMemcpyDeviceToHost, stream));
     MS3_CUDA(cudaStreamSynchronize(stream));
     int64_t total = 0;
     for (int64_t n : counts) total += n;
     times.resize((size_t)total);
     if (total == 0) return;
-    DevBuf dtimes(sizeof(int64_t) * (size_t)total, stream);
-    detect_write<<<gg, 128, 0, stream>>>(d, ncand, cn.as<int64_t>(), ck.as<int32_t>(), use.as<uint8_t>(),
-                                         at.as<int64_t>(), dtimes.as<int64_t>());
-    MS3_LAUNCH_CHECK();
-    MS3_CUDA(cudaMemcpyAsync(times.data(), dtimes.get(), sizeof(int64_t) * (size_t)total, cudaMemcpyDeviceToHost,
-                             stream));
+    MS3_CUDA(cudaMemcpyAsync(times.data(), dtimes, sizeof(int64_t) * (size_t)total, cudaMemcpyDeviceToHost, stream));
     MS3_CUDA(cudaStreamSynchronize(stream));
 }
 

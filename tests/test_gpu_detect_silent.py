@@ -1,6 +1,7 @@
 """The detector's statistics with silent channels and silent stretches, below and above the
-number of (channel, chunk) pairs from which a thread takes each of them: event times equal
-the oracle's, and one silent channel costs hardly more than none."""
+number of (channel, chunk) pairs from which a thread takes each of them and the length and
+number from which segments are long: event times equal the oracle's, and one silent channel
+costs hardly more than none."""
 import numpy as np
 import pytest
 import torch
@@ -25,7 +26,8 @@ def _data(kind, N, M):
 
 
 @pytest.mark.parametrize("kind", ["some", "all", "nan"])
-@pytest.mark.parametrize("N,M,chunk", [(40000, 3, 0), (6300, 65, 100), (6301, 65, 100), (7000, 64, 100), (300, 4096, 0)])
+@pytest.mark.parametrize("N,M,chunk", [(40000, 3, 0), (6300, 65, 100), (6301, 65, 100), (7000, 64, 100), (300, 4096, 0), (14384, 3, 0),
+                                       (14385, 3, 0), (1000, 2730, 0), (1000, 2740, 0)])
 def test_event_times_equal_the_oracles(gpu_lib, ref32, kind, N, M, chunk):
     X = _data(kind, N, M)
     for thr, interval, sign in ((2.0, 25.5, -1), (0.0, 10.0, 0)):
