@@ -43,3 +43,13 @@ def test_norm_batches(gpu_lib, ref32, I, nint):
     out, kept = api.mask_out_artifacts(torch.from_numpy(X).cuda(), threshold=3.0, interval_size=I, return_kept=True)
     np.testing.assert_array_equal(out.cpu().numpy(), ref)
     assert kept == kept_ref
+
+
+@pytest.mark.parametrize("M", [1, 33])
+@pytest.mark.parametrize("nint", [1, 2, 255, 256, 257])  # either side of the limits' own flags
+def test_few_intervals(gpu_lib, ref32, M, nint):
+    X = _data(M, nint * 20 + 3, 20)
+    ref, kept_ref = ref32.mask_out_artifacts(X, threshold=3.0, interval_size=20)
+    out, kept = api.mask_out_artifacts(torch.from_numpy(X).cuda(), threshold=3.0, interval_size=20, return_kept=True)
+    np.testing.assert_array_equal(out.cpu().numpy(), ref)
+    assert kept == kept_ref
