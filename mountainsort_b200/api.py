@@ -125,8 +125,8 @@ _PRECISION = {"plain": _lib.PRECISION_PLAIN, "mixed": _lib.PRECISION_MIXED}
 def whiten(X, quantization_unit=0.0, out=None, stream=None, precision="plain"):
     """ms3.whiten (packages/ms3/p_whiten.cpp:45-206) on an (N, M) array.
     precision "plain" (FP32, parity with the reference) or "mixed"
-    (1e-4 against FP64; it differs from "plain" for int16 output and for
-    matrices whose weights span more than 2^30)."""
+    (1e-4 against FP64; it differs from "plain" for int16 output and, beyond
+    32 channels, for matrices whose weights span more than 2^30)."""
     L = _lib.load()
     X = _as_f32_rows(X)
     N, M = X.shape

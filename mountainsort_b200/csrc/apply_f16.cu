@@ -28,11 +28,12 @@
 // is tiny or zero.  So W decides (split_column): this kernel runs when every weight,
 // after the channels' scales, is at least 2^-30 of its column's largest and of the root
 // of its K-block's sum of squares; then the cut is below 2^-21 of the terms that the output
-// sums, for any x.  Otherwise (an identity, block-diagonal or sparse W) the TF32 kernel
-// runs, which holds each value by itself: both are launched, and the one that W's flag
-// does not name returns at once (300 clips of 32 channels: 3 us of 62).  Whitening matrices of correlated channels have
-// their smallest at 2^-24 (384 channels) to 2^-14 (32); uncorrelated noise, 2^-33 at 200.
-// Only W is looked at, so the same W takes the same kernel in every call and slab.
+// sums, for any x.  Any other W (identity, block-diagonal, sparse) is applied with each
+// value held by itself: up to 32 channels by FP32 FMAs in this kernel (apply_rows), beyond
+// by the TF32 kernel.  Beyond, both kernels are launched and the one that W's flag does not
+// name returns at once (3.5 us).  Whitening matrices of correlated channels have their
+// smallest at 2^-24 (384 channels) to 2^-14 (32); uncorrelated noise, 2^-33 at 200.  Only W
+// is looked at, so the same W takes the same path in every call and slab.
 // A row that holds an infinity or NaN in a K-block, and a column of W that does, come
 // out NaN, as they do from the TF32 split.
 //
@@ -176,6 +177,104 @@ __device__ __forceinline__ float quantize_1e4_any(float x) {
     return (float)__dmul_rn(floor(__dadd_rn(__ddiv_rn((double)x, 0.0001), 0.5)), 0.0001);
 }
 
+// The apply by FP32 FMAs for few channels: a thread forms four outputs of two or four
+// timepoints.  W lies in shared memory as floats, the outputs side by side; timepoints
+// arrive by cp.async, kRowStages - 1 groups ahead.  The line lies where the TF32 kernel in
+// its place is as fast (identity, whole calls: 4 channels x 4M 104 us, TF32 830; 12 x 3M 174
+// and 770; 32 x 1.8M 255 and 253; 64 x 900k 367 and 240); below it that kernel's launch is
+// saved, which small calls notice (300 clips of 32 channels: 57.4 us with it, 53 without).
+constexpr int kRowsM = 32;
+constexpr int kRowStages = 4;
+__host__ __device__ constexpr int row_floats(int M) { return M + 4; }  // of a staged timepoint: no bank conflicts
+__host__ __device__ constexpr int rows_of(int M) { return kThreads / (M / 4); }
+__host__ __device__ constexpr int rows_each(int M) { return M <= 16 ? 2 : 4; }  // of a thread; what fits
+constexpr size_t rows_smem(int M) {
+    return 16 + sizeof(float) * ((size_t)M * M + (size_t)kRowStages * rows_each(M) * rows_of(M) * row_floats(M));
+}
+constexpr bool rows_fit() {
+    for (int M = 4; M <= kRowsM; M += 4)
+        if (rows_smem(M) > smem_bytes(tile_cols(M), tile_cols(M))) return false;
+    return true;
+}
+static_assert(rows_fit(), "shared memory of the FP32 form");
+
+template <int H>
+__device__ __noinline__ void apply_rows(const float* X, const double* __restrict__ W, int M, int64_t N, int64_t ld,
+                                        int round_1e4, float* out) {
+    extern __shared__ uint8_t smem_raw[];
+    constexpr float kMax = 3.402823466e38f;
+    float* ws = reinterpret_cast<float*>(smem_raw + ((0u - tc::smem_u32(smem_raw)) & 15u));
+    float* staged = ws + M * M;
+    const int quads = M / 4, rows = rows_of(M), pitch = row_floats(M);
+    const int r = threadIdx.x / quads, q = threadIdx.x - r * quads;
+    const bool mine = r < rows;
+    const int64_t step = (int64_t)gridDim.x * H * rows;
+    auto bring = [&](int64_t t0, int stage) {
+#pragma unroll
+        for (int h = 0; h < H; h++) {
+            const int64_t t = t0 + h * rows + r;
+            const bool in = t < N;
+            const uint32_t dst = tc::smem_u32(staged + ((size_t)(stage * H + h) * rows + r) * pitch + 4 * q);
+            if (mine)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(X + (in ? t * ld + 4 * q : 0)),
+                             "r"(in ? 16 : 0)
+                             : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    int64_t t0 = (int64_t)blockIdx.x * H * rows;
+#pragma unroll
+    for (int i = 0; i < kRowStages - 1; i++) bring(t0 + i * step, i);
+    for (int i = threadIdx.x; i < M * M; i += kThreads) {  // W^T[m][k] to ws[k][m]
+        const float w = (float)W[i];
+        ws[(i % M) * M + i / M] = fabsf(w) <= kMax ? w : __uint_as_float(0x7FC00000u);
+    }
+    const float4* w = reinterpret_cast<const float4*>(ws) + q;
+    for (int stage = 0; t0 < N; t0 += step, stage = (stage + 1) % kRowStages) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kRowStages - 2) : "memory");
+        __syncthreads();  // the group is here, and every thread is done with the one before
+        bring(t0 + (kRowStages - 1) * step, (stage + kRowStages - 1) % kRowStages);
+        if (!mine) continue;
+        float y[H][4] = {};
+        const float* x0 = staged + ((size_t)stage * H * rows + r) * pitch;  // + h rows pitch: this thread's timepoints
+        const int next = rows * pitch;
+#pragma unroll 2
+        for (int c = 0; c < quads; c++) {
+            float4 v[H];
+#pragma unroll
+            for (int h = 0; h < H; h++) v[h] = *reinterpret_cast<const float4*>(x0 + h * next + 4 * c);
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float4 u = w[(4 * c + i) * quads];
+#pragma unroll
+                for (int h = 0; h < H; h++) {
+                    const float x = i == 0 ? v[h].x : i == 1 ? v[h].y : i == 2 ? v[h].z : v[h].w;
+                    y[h][0] = __fmaf_rn(x, u.x, y[h][0]);
+                    y[h][1] = __fmaf_rn(x, u.y, y[h][1]);
+                    y[h][2] = __fmaf_rn(x, u.z, y[h][2]);
+                    y[h][3] = __fmaf_rn(x, u.w, y[h][3]);
+                }
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < H; h++) {
+            const int64_t t = t0 + h * rows + r;
+            if (t >= N) continue;
+            // an infinity or NaN in the row leaves no output finite: all of them become NaN
+            if (!(fabsf(y[h][0]) <= kMax) && !(fabsf(y[h][1]) <= kMax) && !(fabsf(y[h][2]) <= kMax) && !(fabsf(y[h][3]) <= kMax))
+                for (int k = 0; k < M; k++)
+                    if (!(fabsf(x0[h * next + k]) <= kMax)) y[h][0] = y[h][1] = y[h][2] = y[h][3] = __uint_as_float(0x7FC00000u);
+            if (round_1e4) {
+#pragma unroll
+                for (int j = 0; j < 4; j++) y[h][j] = quantize_1e4_any(y[h][j]);
+            }
+            if (MS3_IN_BOUNDS(t * ld + 4 * q + 3, (N - 1) * ld + M, 305))
+                *reinterpret_cast<float4*>(out + t * ld + 4 * q) = make_float4(y[h][0], y[h][1], y[h][2], y[h][3]);
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
 // COLS: columns of a drain thread, a multiple of 16 that covers them; instances for few
 // columns are short enough for the instruction cache.
 template <int COLS>
@@ -183,11 +282,14 @@ __global__ void __launch_bounds__(kThreads, 1)
     apply_f16_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmWh,
                      const __grid_constant__ CUtensorMap tmWl, const __grid_constant__ CUtensorMap tmOut, int64_t M,
                      int64_t N, int BN, int ncb, int64_t ntiles, const float* __restrict__ in_scale,
-                     const float* __restrict__ col_scale, const int* __restrict__ wide, int round_1e4,
-                     int* __restrict__ err) {
-    if (*wide) return;  // the TF32 kernel's
+                     const float* __restrict__ col_scale, const int* __restrict__ wide, const float* X,
+                     const double* __restrict__ W, int64_t ld, float* out, int round_1e4, int* __restrict__ err) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    if (*wide) {  // beyond kRowsM the TF32 kernel's
+        if (COLS <= kRowsM && M <= kRowsM) apply_rows<rows_each(COLS)>(X, W, (int)M, N, ld, round_1e4, out);
+        return;
+    }
     const uint32_t w_bytes = (uint32_t)BN * 128u;  // one of W_h, W_l
     uint8_t* xs = smem;
     uint8_t* ws = xs + kXStages * kXBytes;
@@ -483,7 +585,7 @@ __device__ __forceinline__ double inverse_pow2(float s) {
 // the other, the scales, and the flag for a W that the other takes.
 struct SplitW {
     __half *hi, *lo;        // [M][Kp]
-    float *hi32, *lo32;     // [M][M]
+    float *hi32, *lo32;     // [M][M], or null (kRowsM)
     float *in_scale, *col_scale;
     int *wide, *err;        // err: null, or cleared
 };
@@ -552,7 +654,7 @@ __device__ __forceinline__ void split_column(const double* __restrict__ w, int64
         const __half h = __double2half(x);
         hi[k] = h;
         lo[k] = __double2half((x - (double)__half2float(h)) * (double)kLowScale);
-        if (k < M) {
+        if (o.hi32 && k < M) {
             const float h32 = __uint_as_float(tc::cvt_rna_tf32((float)v));
             o.hi32[m * M + k] = h32;
             o.lo32[m * M + k] = __uint_as_float(tc::cvt_rna_tf32((float)(v - (double)h32)));
@@ -686,7 +788,7 @@ void apply_whitening_f16(const float* X, int64_t M, int64_t N, const double* W, 
     const int64_t n_in = ceil_div(M, kKB) * kKB;
     const size_t n_scales = (size_t)n_in + (size_t)ncb * (size_t)BN;
     auto padded = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
-    const size_t half_bytes = padded((size_t)(M * Kp) * sizeof(__half)), tf32_bytes = padded((size_t)(M * M) * sizeof(float));
+    const size_t half_bytes = padded((size_t)(M * Kp) * sizeof(__half)), tf32_bytes = M > kRowsM ? padded((size_t)(M * M) * sizeof(float)) : 0;
     DevBuf buf(2 * half_bytes + 2 * tf32_bytes + n_scales * sizeof(float) + 256, stream);
     SplitW w;
     char* at = buf.as<char>();
@@ -695,6 +797,7 @@ void apply_whitening_f16(const float* X, int64_t M, int64_t N, const double* W, 
     w.hi32 = reinterpret_cast<float*>(at += half_bytes);
     w.lo32 = reinterpret_cast<float*>(at += tf32_bytes);
     w.in_scale = reinterpret_cast<float*>(at += tf32_bytes);
+    if (!tf32_bytes) w.hi32 = w.lo32 = nullptr;
     w.col_scale = w.in_scale + n_in;
     w.wide = reinterpret_cast<int*>(w.in_scale + n_scales);
     w.err = ext_err ? nullptr : w.wide + 1;  // the call's own flag: cleared with the preparation of W
@@ -725,9 +828,12 @@ void apply_whitening_f16(const float* X, int64_t M, int64_t N, const double* W, 
                 : cols <= 64 ? apply_f16_kernel<64>
                              : apply_f16_kernel<96>;
     kern<<<(unsigned)std::min<int64_t>(ntiles, nsm), kThreads, sm, stream>>>(
-        mx, mh, ml, mo, M, N, BN, ncb, ntiles, w.in_scale, w.col_scale, w.wide, round_1e4 ? 1 : 0, err);
+        mx, mh, ml, mo, M, N, BN, ncb, ntiles, w.in_scale, w.col_scale, w.wide, X, W, ld, static_cast<float*>(out),
+        round_1e4 ? 1 : 0, err);
     MS3_LAUNCH_CHECK();
-    apply_tc_launch(X, M, N, ld, w.hi32, w.lo32, /*quantization_unit=*/0.0, drain, round_1e4, out, err, w.wide, stream);
+    if (M > kRowsM)
+        apply_tc_launch(X, M, N, ld, w.hi32, w.lo32, /*quantization_unit=*/0.0, drain, round_1e4, out, err, w.wide,
+                        stream);
     if (ext_err) return;  // the caller checks the flag once for many calls
     if (host_err) {  // the caller looks at it after its own synchronisation
         MS3_CUDA(cudaMemcpyAsync(host_err, err, sizeof(int), cudaMemcpyDeviceToHost, stream));

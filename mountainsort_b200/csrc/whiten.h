@@ -87,9 +87,9 @@ void whitening_matrix_device(const double* XXt, int64_t M, double* W, double* co
 
 // out = quantize(W^T x) per timepoint; out float32, or int16 when
 // quantization_unit > 0.  Float output on the tensor cores from 11-bit halves where
-// apply_f16_supported and W's weights span less than 2^30; otherwise three TF32 products,
-// drained per K-block or, mixed, accumulated over K, where apply_tc_supported; otherwise
-// FP32 FMA.
+// apply_f16_supported and W's weights span less than 2^30 (or M is at most 32: else FP32
+// FMA there); otherwise three TF32 products, drained per K-block or, mixed, accumulated
+// over K, where apply_tc_supported; otherwise FP32 FMA.
 // err: optional device flag raised by a timed-out tensor-core pipeline; when
 // null the call keeps one of its own and copies it to host_err on the stream, or,
 // when that is null too, checks it itself (synchronising the stream).
@@ -117,7 +117,8 @@ void apply_tc_launch(const float* X, int64_t M, int64_t N, int64_t ld, const flo
 
 // Tensor-core apply with float output from halves of 11 bits (three products,
 // round-to-nearest sums per 64 channels): both precision forms, for a W whose weights
-// allow it (apply_f16.cu); any other W goes through apply_tc_launch, drained or not.
+// allow it (apply_f16.cu); any other W takes FP32 FMAs up to 32 channels and
+// apply_tc_launch, drained or not, beyond.
 bool apply_f16_supported(const float* X, int64_t M, int64_t N, const void* out, int64_t ld);
 void apply_whitening_f16(const float* X, int64_t M, int64_t N, const double* W, bool drain, void* out,
                          cudaStream_t stream, int* err, bool round_1e4, int64_t ld, int* host_err);
