@@ -48,7 +48,7 @@
 // straight from registers slower (498 against 462 us), a single accumulation over K
 // would be less exact than TF32 with drains.
 // 384 channels x 300k: 590 us with TF32 (128 x 128 tiles, 32-wide blocks, FP64 rounding),
-// now 399; 200 x 1.5M: 1253 (undrained) and 921; 32 x 1.8M: 213 and 125.
+// now 407; 200 x 1.5M: 1253 (undrained) and 944; 32 x 1.8M: 213 and 124.
 //
 // A persistent CTA per SM walks tiles of 128 timepoints x BN channels (BN <= 192):
 //   warp 0       TMA: X (two 128 x 32 float boxes) into a ring of kXStages, W_h and

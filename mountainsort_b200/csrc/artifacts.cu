@@ -12,7 +12,7 @@
 //         beyond the last whole interval (never written by the reference).
 //
 // Four kernels: norms (one thread per channel and interval), per-channel limits,
-// interval flags, and a masked copy.
+// interval flags (a few by the limits kernel), and a masked copy.
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -39,7 +39,7 @@
 // (values rounded to 1e-4: none; unrounded floats: up to a third of the segments).  A
 // segment of zeros adds nothing.
 // 64 channels x 1.8M timepoints in one chunk, whole call, serially and by segments: 75 and
-// 1.1 ms for values rounded to 1e-4, 10 ms for unrounded ones, 31 ms for values over 40
+// 1.1 ms for values rounded to 1e-4, 9 ms for unrounded ones, 26 ms for values over 40
 // octaves.
 #include <cuda_runtime.h>
 

@@ -518,7 +518,7 @@ __global__ void __launch_bounds__(kPcaThreads) pca_cluster(const double* __restr
 //
 // CS = 1 (M <= 128): one CTA; rows meet in shared memory, one block barrier a
 // step.  344 us at 32 channels and 1468 us at 128 with the 8-CTA cluster that this
-// replaces; now 146 us and 1130 us.
+// replaces; now 139 us and 1097 us.
 // CS = 16 (M > 128): sixteen CTAs of NW warps; row m belongs to CTA m % CS, so
 // every CTA owns rows.  A CTA gathers its rows in shared memory (the step's one
 // block barrier) and each warp stores them to its share of the sixteen CTAs with
@@ -532,7 +532,7 @@ __global__ void __launch_bounds__(kPcaThreads) pca_cluster(const double* __restr
 // under a microsecond, less than a suspended wait takes to wake) and are bounded
 // (error flag g_pca_timeout).  Eight CTAs of 16 warps and 3 rows, with division
 // and vector handed round through shared memory, took 8230 us at 384 channels and
-// 3023 us at 200; this takes 4030 us and 1640 us.
+// 3023 us at 200; this takes 4107 us and 1624 us.
 __device__ int g_pca_timeout;  // set when an exchange wait gave up (checked by the host)
 
 __device__ __noinline__ double plain_quotient(double y, double b) { return y / b; }
